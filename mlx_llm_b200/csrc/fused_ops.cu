@@ -8,6 +8,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "layer_kernels.h"
 
 namespace {
 
@@ -145,50 +146,78 @@ __global__ void residual_add_f32_kernel(const float* __restrict__ y, int64_t n, 
     }
 }
 
-// Greedy argmax over bf16 logits, first maximum wins (src/primitives/sampler.rs:221-241).
-__global__ void argmax_kernel(const uint16_t* __restrict__ logits, int vocab, int32_t* __restrict__ out) {
-    const uint16_t* row = logits + (size_t)blockIdx.x * vocab;
+// Greedy argmax over the rows of bf16 or f32 logits, first maximum wins (src/primitives/sampler.rs:221-241); rows with no value above
+// -inf give index 0, as a host scan starting from best = -inf, index 0 does.
+// Bound by the latency of its loads: a row is a few hundred KB, which one block reads in 32 dependent rounds.  A cluster of eight blocks
+// takes a row in 16-byte pieces, four rounds a thread, and the blocks hand their maxima to the first one through its shared memory.
+// 128256 bf16 logits: 54 us with a block per row and 2-byte loads (one row as well as 97), now 4 us for one row, 11 us for 97.
+constexpr int kArgmaxBlocks = 8;
+template <typename T>
+__global__ void __cluster_dims__(kArgmaxBlocks, 1, 1) __launch_bounds__(512)
+    argmax_kernel(const T* __restrict__ logits, int64_t ld, int vocab, int32_t* __restrict__ out) {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");  // (waited for before another block's shared memory is written)
+    pdl_wait();
+    constexpr int V = 16 / sizeof(T);
+    const int part = blockIdx.x % kArgmaxBlocks, first = part * blockDim.x + threadIdx.x, stride = kArgmaxBlocks * blockDim.x;
+    const T* row = logits + (size_t)(blockIdx.x / kArgmaxBlocks) * ld;
     float best = -INFINITY;
     int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
-        const float v = bf2f(row[i]);
-        if (v > best) {  // strictly greater: within a thread indices ascend, so the first max is kept
-            best = v;
-            bi = i;
-        }
-    }
-    __shared__ float sv[32];
-    __shared__ int si[32];
+    auto value = [](T x) {
+        if constexpr (sizeof(T) == 2)
+            return bf2f(x);
+        else
+            return x;
+    };
+    auto step = [&](float v, int i) {
+        if (v > best) best = v, bi = i;  // strictly greater: a thread's indices ascend, so its first maximum is kept
+    };
+    const int whole = ((uintptr_t)row & 15) == 0 ? vocab / V : 0;  // 16-byte pieces, where the row is aligned for them
+#pragma unroll 4
+    for (int i = first; i < whole; i += stride) {
+        uint4 raw = *reinterpret_cast<const uint4*>(row + (size_t)i * V);
+        const T* v = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(kFull, best, o);
-        const int oi = __shfl_xor_sync(kFull, bi, o);
-        if (ov > best || (ov == best && oi < bi)) {
-            best = ov;
-            bi = oi;
-        }
+        for (int j = 0; j < V; j++) step(value(v[j]), i * V + j);
     }
-    if ((threadIdx.x & 31) == 0) {
-        sv[threadIdx.x >> 5] = best;
-        si[threadIdx.x >> 5] = bi;
-    }
+    for (int i = whole * V + first; i < vocab; i += stride) step(value(row[i]), i);
+    auto take = [&](float ov, int oi) {
+        if (ov > best || (ov == best && oi < bi)) best = ov, bi = oi;
+    };
+    __shared__ float sv[16], cv[kArgmaxBlocks];
+    __shared__ int si[16], ci[kArgmaxBlocks];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) take(__shfl_xor_sync(kFull, best, o), __shfl_xor_sync(kFull, bi, o));
+    if ((threadIdx.x & 31) == 0) sv[threadIdx.x >> 5] = best, si[threadIdx.x >> 5] = bi;
+    asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32) {
-        const int nw = blockDim.x >> 5;
-        best = threadIdx.x < nw ? sv[threadIdx.x] : -INFINITY;
-        bi = threadIdx.x < nw ? si[threadIdx.x] : 0x7fffffff;
+        best = threadIdx.x < 16 ? sv[threadIdx.x] : -INFINITY;
+        bi = threadIdx.x < 16 ? si[threadIdx.x] : 0x7fffffff;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(kFull, best, o);
-            const int oi = __shfl_xor_sync(kFull, bi, o);
-            if (ov > best || (ov == best && oi < bi)) {
-                best = ov;
-                bi = oi;
-            }
+        for (int o = 8; o > 0; o >>= 1) take(__shfl_xor_sync(kFull, best, o), __shfl_xor_sync(kFull, bi, o));
+        if (threadIdx.x == 0) {
+            uint32_t v, i;
+            asm("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(v) : "r"(smem_u32(cv + part)));
+            asm("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(i) : "r"(smem_u32(ci + part)));
+            asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(v), "f"(best) : "memory");
+            asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(i), "r"(bi) : "memory");
         }
-        // all logits -inf or NaN: index 0, as a host scan starting from best = -inf, index 0 gives
-        if (threadIdx.x == 0) out[blockIdx.x] = bi == 0x7fffffff ? 0 : bi;
     }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    if (part == 0 && threadIdx.x == 0) {
+        best = -INFINITY, bi = 0x7fffffff;
+#pragma unroll
+        for (int j = 0; j < kArgmaxBlocks; j++) take(cv[j], ci[j]);
+        out[blockIdx.x / kArgmaxBlocks] = bi == 0x7fffffff ? 0 : bi;
+    }
+}
+template <typename T>
+int32_t launch_argmax(b2_ctx* ctx, const T* logits, int64_t ld, int rows, int vocab, int32_t* out) {
+    if (rows <= 0) return B2_OK;
+    B2_CUDA(b2_launch_pdl(ctx->pdl_consumers, argmax_kernel<T>, dim3((unsigned)rows * kArgmaxBlocks), dim3(512), 0, ctx->stream, logits, ld, vocab, out));
+    B2_LAUNCHED(ctx);
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
 }
 
 // Standalone dequantize / unpack of the MLX affine format (src/primitives/quant.rs:73-82).
@@ -309,11 +338,10 @@ int32_t b2_residual_add_f32_launch(b2_ctx* ctx, const float* y, int64_t n, uint1
     return B2_OK;
 }
 int32_t b2_argmax_launch(b2_ctx* ctx, const uint16_t* logits, int rows, int vocab, int32_t* out) {
-    if (rows <= 0) return B2_OK;
-    argmax_kernel<<<rows, 1024, 0, ctx->stream>>>(logits, vocab, out);
-    B2_LAUNCHED(ctx);
-    B2_CUDA(cudaGetLastError());
-    return B2_OK;
+    return launch_argmax(ctx, logits, vocab, rows, vocab, out);
+}
+int32_t b2_argmax_f32_launch(b2_ctx* ctx, const float* logits, int ld, int rows, int vocab, int32_t* out) {
+    return launch_argmax(ctx, logits, ld, rows, vocab, out);
 }
 int32_t b2_dequantize_launch(b2_ctx* ctx, const uint32_t* packed, const uint16_t* scales, const uint16_t* biases, int64_t rows,
                              int64_t in_dim, int bits, uint16_t* out) {

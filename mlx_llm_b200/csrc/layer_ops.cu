@@ -516,37 +516,6 @@ __global__ void __launch_bounds__(256) linear_f32_blocked_kernel(const float* __
         if (t0 + ty * 4 + i < M) y[(size_t)(t0 + ty * 4 + i) * ldy + j] = acc[i];
 }
 
-__global__ void argmax_rows_f32_kernel(const float* __restrict__ logits, int ld, int vocab, int32_t* __restrict__ out) {
-    pdl_wait();
-    __shared__ float bv[32];
-    __shared__ int bi[32];
-    const float* row = logits + (size_t)blockIdx.x * ld;
-    float best = -INFINITY;
-    int idx = 0x7fffffff;
-    for (int i = threadIdx.x * 4; i < vocab; i += blockDim.x * 4) {  // (ld is a multiple of 128) a thread's ids ascend: its first maximum is kept
-        const float4 v = *reinterpret_cast<const float4*>(row + i);
-        if (v.x > best) best = v.x, idx = i;
-        if (i + 1 < vocab && v.y > best) best = v.y, idx = i + 1;
-        if (i + 2 < vocab && v.z > best) best = v.z, idx = i + 2;
-        if (i + 3 < vocab && v.w > best) best = v.w, idx = i + 3;
-    }
-    auto take = [&](float ov, int oi) {
-        if (ov > best || (ov == best && oi < idx)) best = ov, idx = oi;
-    };
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) take(__shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, idx, o));
-    if ((threadIdx.x & 31) == 0) bv[threadIdx.x >> 5] = best, bi[threadIdx.x >> 5] = idx;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int nw = blockDim.x >> 5;
-        best = threadIdx.x < nw ? bv[threadIdx.x] : -INFINITY;
-        idx = threadIdx.x < nw ? bi[threadIdx.x] : 0x7fffffff;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) take(__shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, idx, o));
-        if (threadIdx.x == 0) out[blockIdx.x] = idx == 0x7fffffff ? 0 : idx;
-    }
-}
-
 int threads_for(int n, int per, int cap) {
     int t = (n + per - 1) / per;
     t = (t + 31) / 32 * 32;
@@ -670,12 +639,6 @@ int32_t b2_zero_cols_launch(b2_ctx* ctx, bool f32, void* x, int ldx, int c0, int
 int32_t b2_linear_f32_launch(b2_ctx* ctx, const float* x, int ldx, const float* w, int M, int N, int K, float* y, int ldy) {
     if (M <= 0) return B2_OK;
     B2_CUDA(b2_launch_pdl(ctx->pdl_consumers, linear_f32_blocked_kernel, dim3((N + 31) / 32, (M + 31) / 32), dim3(256), 0, ctx->stream, x, ldx, w, M, N, K, y, ldy));
-    B2_LAUNCHED(ctx);
-    return B2_OK;
-}
-int32_t b2_argmax_f32_launch(b2_ctx* ctx, const float* logits, int ld, int rows, int vocab, int32_t* out) {
-    if (rows <= 0) return B2_OK;
-    B2_CUDA(b2_launch_pdl(ctx->pdl_consumers, argmax_rows_f32_kernel, dim3(rows), dim3(1024), 0, ctx->stream, logits, ld, vocab, out));
     B2_LAUNCHED(ctx);
     return B2_OK;
 }

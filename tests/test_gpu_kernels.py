@@ -394,3 +394,21 @@ def test_prefill_attention_rising_scores_hd128(env):
                               case["scale"])
     ok, err = H.close_bf16_out(out.download(), ref)
     assert ok, f"max-abs {err}"
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 1), (3, 7), (2, 4095), (5, 32768), (2, 32771), (97, 1000)])
+def test_argmax_sizes(env, rows, vocab):
+    """Rows of every alignment, whole pieces and remainders; each row's maximum twice, values that are not numbers beside it."""
+    ctx, K, orc = env
+    rng = np.random.default_rng(vocab)
+    values = rng.standard_normal((rows, vocab)).astype(np.float32)
+    for r in range(rows):
+        at = np.sort(rng.integers(0, vocab, 2))
+        values[r, at] = 9.0
+        if at[0] > 0:
+            values[r, 0] = np.nan
+    logits = H.f32_to_bf16_np(values)
+    out = ctx.empty((rows,), np.int32)
+    K.argmax(ctx, ctx.buf(logits), rows, vocab, out)
+    ctx.sync()
+    assert out.download().tolist() == [int(np.nanargmax(v)) for v in values]
