@@ -169,15 +169,23 @@ int32_t set_local_dims(b2_model* m, b2_tp_group* tp) {
     return B2_OK;
 }
 
-// The large-M projection kernel reads scale and bias of 32 feature rows at one K group in one instruction: a second
-// copy of both, transposed and interleaved, makes that one line instead of 64.  (Not counted in weight_bytes: it is a
+// The projection kernels take scale and bias of a tile's feature rows at one K group as consecutive words: a second
+// copy of both, transposed and interleaved, makes that one line for 32 rows instead of 64.  (Not counted in weight_bytes: it is a
 // derived layout, 1/9 of the packed 4-bit codes.)
 static int32_t build_sbt(b2_model* m, Proj& p) {
     if (p.bits == 0 || p.sbt) return B2_OK;
     const int G = p.K / 64;
-    B2_CUDA(cudaMalloc((void**)&p.sbt, (size_t)p.N * G * 4));
-    m->allocs.push_back(p.sbt);
-    return b2_gemm_build_sbt(m->ctx, p.scales, p.biases, p.N, G, p.sbt);
+    uint32_t* table = nullptr;
+    int usable = 0;
+    B2_CUDA(cudaMalloc((void**)&table, (size_t)p.N * G * 4));
+    const int32_t rc = b2_gemm_build_sbt(m->ctx, p.scales, p.biases, p.N, G, table, &usable);
+    if (rc != B2_OK || !usable) {
+        cudaFree(table);
+        return rc;
+    }
+    p.sbt = table;
+    m->allocs.push_back(table);
+    return B2_OK;
 }
 
 int32_t finish_model(b2_model* m) {

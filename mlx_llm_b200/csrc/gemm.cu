@@ -272,7 +272,9 @@ int32_t b2_gemm_launch(b2_ctx* ctx, const GemmParams& p) {
         B2_REQUIRE(p.K % 64 == 0, B2_ERR_UNSUPPORTED, "gemm: K must be a multiple of the group size");
         B2_REQUIRE(p.bits == 4 || p.bits == 8, B2_ERR_UNSUPPORTED, "gemm: bits must be 4 or 8");
     }
-    // Up to 32 tokens the weight-streaming kernel wins; from 33 on the tcgen05 kernel does where its tiling fits (one
+    // Up to 16 (Q4) or 32 tokens the ring kernel where the weights are dense or come with their table; figures in gemm_ring.cu.
+    if (ctx->use_tc && b2_gemm_ring_eligible(ctx, p)) return b2_gemm_ring_launch(ctx, p);
+    // Otherwise up to 32 tokens the weight-streaming kernel wins; from 33 on the tcgen05 kernel does where its tiling fits (one
     // 16-token-granular block costs it the same as a full one, while the streaming kernel's cost grows with the tokens);
     // the streaming kernel keeps 33..64 tokens for the shapes the tcgen05 tiling does not take.
     const bool tc_ok = ctx->use_tc && b2_gemm_tc_eligible(p);

@@ -375,14 +375,9 @@ int32_t launch_stream(b2_ctx* ctx, const GemmParams& p) {
     const int smem = 2 * NT * 8 * XS_STRIDE;
     B2_SMEM_ONCE(ctx, (gemm_stream_kernel<WK, NT, EPI>), smem);
     const int row_tiles = p.N / ROWS_PER_CTA;
-    const int chunks = p.K / KC;
-    // K ranges: enough CTAs for every slot of the machine, at least two chunks per range
-    int splits = (4 * ctx->sm_count + row_tiles - 1) / row_tiles;  // four CTAs fit an SM (registers): fill them all
-    if (splits > chunks / 2) splits = chunks / 2;
-    if (splits < 1) splits = 1;
-    const int chunks_per = (chunks + splits - 1) / splits;
-    splits = (chunks + chunks_per - 1) / chunks_per;
-    StreamExtra ex{splits, chunks_per * KC, nullptr, nullptr};
+    const RangePlan cut = b2_gemm_stream_ranges(ctx, p.N, p.K);
+    const int splits = cut.ranges;
+    StreamExtra ex{splits, cut.k_per_range, nullptr, nullptr};
     if (splits > 1) {
         const size_t bytes = (size_t)splits * p.M * p.N * sizeof(float);
         if (bytes > ctx->tc_partial_bytes) {
@@ -443,6 +438,16 @@ int32_t dispatch_nt(b2_ctx* ctx, const GemmParams& p) {
 }
 
 }  // namespace
+
+RangePlan b2_gemm_stream_ranges(b2_ctx* ctx, int N, int K) {
+    // enough CTAs for every slot of the machine, at least two chunks per range; four CTAs fit an SM (registers)
+    const int row_tiles = N / ROWS_PER_CTA, chunks = K / KC;
+    int splits = (4 * ctx->sm_count + row_tiles - 1) / row_tiles;
+    if (splits > chunks / 2) splits = chunks / 2;
+    if (splits < 1) splits = 1;
+    const int chunks_per = (chunks + splits - 1) / splits;
+    return RangePlan{(chunks + chunks_per - 1) / chunks_per, chunks_per * KC};
+}
 
 bool b2_gemm_stream_eligible(const GemmParams& p) {
     return p.M >= 1 && p.M <= 64 && p.N % ROWS_PER_CTA == 0 && p.K % KC == 0 && p.ldx % 4 == 0 && ((uintptr_t)p.x & 7) == 0 &&

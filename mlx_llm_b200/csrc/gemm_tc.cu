@@ -764,13 +764,18 @@ int32_t get_map(b2_ctx* ctx, const void* ptr, uint64_t rows, uint64_t k, uint64_
     return B2_OK;
 }
 
-__global__ void sbt_build_kernel(const uint16_t* __restrict__ scales, const uint16_t* __restrict__ biases, int N, int G, uint32_t* __restrict__ sbt) {
+__global__ void sbt_build_kernel(const uint16_t* __restrict__ scales, const uint16_t* __restrict__ biases, int N, int G, uint32_t* __restrict__ sbt,
+                                 int* __restrict__ wide) {
     // 32 x 32 tiles through shared memory: coalesced reads along the groups of a row, coalesced writes along the rows
     __shared__ uint32_t tile[32][33];
     const int g0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         const int n = n0 + r, g = g0 + threadIdx.x;
-        if (n < N && g < G) tile[r][threadIdx.x] = (uint32_t)scales[(size_t)n * G + g] | ((uint32_t)biases[(size_t)n * G + g] << 16);
+        if (n < N && g < G) {
+            const uint32_t scale = scales[(size_t)n * G + g];
+            if ((scale & 0x7f80u) >= 0x5000u) *wide = 1;  // 2^33 and more
+            tile[r][threadIdx.x] = scale | ((uint32_t)biases[(size_t)n * G + g] << 16);
+        }
     }
     __syncthreads();
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -871,10 +876,17 @@ int32_t dispatch_pair(b2_ctx* ctx, const GemmParams& p, int* err) {
 
 }  // namespace
 
-int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev) {
-    sbt_build_kernel<<<dim3((unsigned)((G + 31) / 32), (unsigned)((N + 31) / 32)), dim3(32, 8), 0, ctx->stream>>>(scales_dev, biases_dev, N, G, sbt_dev);
+int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev, int* usable) {
+    void* wide = nullptr;
+    int found = 0;
+    B2_CHECK(b2_ctx_scratch(ctx, sizeof(int), &wide));
+    B2_CUDA(cudaMemsetAsync(wide, 0, sizeof(int), ctx->stream));
+    sbt_build_kernel<<<dim3((unsigned)((G + 31) / 32), (unsigned)((N + 31) / 32)), dim3(32, 8), 0, ctx->stream>>>(scales_dev, biases_dev, N, G, sbt_dev, (int*)wide);
     B2_LAUNCHED(ctx);
     B2_CUDA(cudaGetLastError());
+    B2_CUDA(cudaMemcpyAsync(&found, wide, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    B2_CUDA(cudaStreamSynchronize(ctx->stream));
+    *usable = !found;
     return B2_OK;
 }
 

@@ -54,7 +54,7 @@ struct GemmParams {
     // sum to the rank that will add it up.  f32_chunk is a multiple of 4.
     float* out_f32_by_chunk[8];
     int f32_chunk;
-    // Optional (quantized, tcgen05 path): sbt[g * N + n] = scale(n, g) | bias(n, g) << 16, the scales and biases
+    // Optional (quantized): sbt[g * N + n] = scale(n, g) | bias(n, g) << 16, the scales and biases
     // transposed and interleaved so that the 32 feature rows of a warp read one 128-byte line per K group.
     const uint32_t* sbt;
 };
@@ -75,11 +75,21 @@ int32_t b2_gemm_launch(b2_ctx* ctx, const GemmParams& p);
 // weight-streaming kernel for up to 64 tokens (gemm_stream.cu): taken by b2_gemm_launch when eligible.
 bool b2_gemm_stream_eligible(const GemmParams& p);
 int32_t b2_gemm_stream_launch(b2_ctx* ctx, const GemmParams& p);
+// The K ranges that a projection of few tokens is summed in: each on its own, then one after the other.  Both kernels keep to them,
+// so that their results are the same bits.
+struct RangePlan {
+    int ranges, k_per_range;  // (the last range may be shorter)
+};
+RangePlan b2_gemm_stream_ranges(b2_ctx* ctx, int N, int K);
+// up to 32 tokens (Q4: 16), for weights that come with a transposed table of scales and biases, or are dense (gemm_ring.cu)
+bool b2_gemm_ring_eligible(b2_ctx* ctx, const GemmParams& p);
+int32_t b2_gemm_ring_launch(b2_ctx* ctx, const GemmParams& p);
 // tcgen05 / TMEM path, CTA-pair form (gemm_tc.cu): taken by b2_gemm_launch when eligible.
 bool b2_gemm_tc_eligible(const GemmParams& p);
 int32_t b2_gemm_tc_launch(b2_ctx* ctx, const GemmParams& p);
-// fills sbt (N * G words) from scales / biases [N, G] (see GemmParams::sbt); enqueued on the context's stream
-int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev);
+// Fills sbt (N * G words) from scales / biases [N, G] (see GemmParams::sbt) and waits for it.  *usable is 0 when a scale is 2^33 or
+// more in size, infinite or not a number: the kernels that take the table scale its words by powers of two (gemm_ring.cu).
+int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev, int* usable);
 
 // ---- elementwise / normalisation / embedding / sampling (fused_ops.cu) ---------------------------
 // out = rmsnorm(x) * w, one row per token; rows gathered through `row_idx` when non-null.

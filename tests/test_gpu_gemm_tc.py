@@ -121,3 +121,31 @@ def test_stream_matches_tile_kernel(env):
         outs.append(y.download())
     _lib.check(_lib.load().b2_ctx_set_tensor_path(ctx.h, 1))
     assert np.abs(outs[0] - outs[1]).max() <= 1e-4
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 128, 256), (8, 128, 14336), (9, 2048, 2048), (16, 384, 7936), (17, 256, 512), (31, 1024, 2048), (32, 20480, 1024), (3, 77824, 256)])
+def test_ring_gemm_vs_oracle(env, m, n, k):
+    """Dense weights take the ring kernel up to 32 tokens: one K range and several, ranges of unequal length, blocks with several ranges,
+    clusters of every occurring size, more tiles than the machine holds at once."""
+    ctx, K, orc, _lib = env
+    rng = np.random.default_rng(m + n + k)
+    x = H.f32_to_bf16_np(rng.standard_normal((m, k)).astype(np.float32))
+    w = H.f32_to_bf16_np(rng.standard_normal((n, k)).astype(np.float32) * 0.03)
+    yb, yf = ctx.empty((m, n), np.uint16), ctx.empty((m, n), np.float32)
+    K.linear(ctx, ctx.buf(x), ctx.buf(w), m, n, k, yb, yf)
+    rf, _ = orc.linear(x, w)
+    ctx.sync()
+    assert np.abs(yf.download() - rf).max() <= 2e-3
+    assert H.close_bf16_out(yb.download(), rf)[0]
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("batch", [1, 8, 9, 16, 23])
+def test_ring_gemm_quantized_in_a_model(env, bits, batch):
+    """Quantized weights take the ring kernel where a model holds their table: single-token steps of a small model against the oracle."""
+    from mlx_llm_b200 import engine
+    from tests.test_gpu_real_shapes import LLAMA_CUT, run_schedule
+
+    ctx, K, orc, _lib = env
+    cfg = dict(LLAMA_CUT, layers=1, hidden=512, heads=4, kv_heads=1, inter=2816, vocab=1024, quant_bits=bits)
+    run_schedule((ctx, engine, K, orc), cfg, [[(i, 2 + i % 3) for i in range(batch)], [(i, 1) for i in range(batch)]])
