@@ -8,7 +8,7 @@
 // costs and the fixed time of a launch.
 //   * A stage, 128 feature rows x 128 bytes, comes in by one TMA copy, with its scales and biases (from the transposed table) as bulk
 //     copies on the same barrier: no address arithmetic, no load per row, 130 KB in flight on an SM without a register.
-//   * A code becomes a bf16 weight in little more than one instruction (below), two 16-byte shared-memory loads feed a row's 32 codes
+//   * A code becomes a bf16 weight in little more than one instruction (dequant.cuh), two 16-byte shared-memory loads feed a row's 32 codes
 //     and the activations of two MMA steps.  Both are free of bank conflicts: MMA row g is feature row 4 (g & 1) + g / 2, so that the
 //     rows of a quarter-warp lie in different halves of the 128-byte swizzle, and the activations are laid out as [8 K][thread of a
 //     row group] with 64 bytes more than a multiple of 128 per token.
@@ -24,6 +24,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "dequant.cuh"
 #include "kernels.h"
 #include "tc5.cuh"
 
@@ -51,21 +52,6 @@ struct Ring {
     static_assert(STAGES >= 3 && SUMS <= STAGES * STAGE);
 };
 
-__device__ __forceinline__ uint32_t fma_bf2(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.bf16x2 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t mul_bf2(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.bf16x2 %0, %1, %2;\n" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -77,23 +63,6 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     return v;
 }
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(kConsumers) : "memory"); }
-
-// Codes become weights without a conversion: an unsigned byte c in the low bits of a bf16, with nothing above it, IS the number
-// c 2^-133 (up to 127 a subnormal, from 128 on the exponent's lowest bit takes over where they end).  One fma with scale 2^93 and
-// bias 2^-40 then gives bf16(c scale + bias) 2^-40 with the one rounding that the format asks for, and the sums are scaled back
-// at the end.  For a nibble in bits 4-7 the factor is 2^4 smaller.  Exact for scales below 2^33 (others get no table, see
-// b2_gemm_build_sbt) and weights above 2^-86.  Against masking into 128 + c and subtracting: 9 instructions for 8 codes instead of 15.
-constexpr uint32_t kByteUnit = 0x2b806e00u;    // (2^93, 2^-40) for (scale, bias)
-constexpr uint32_t kNibbleUnit = 0x2b806c00u;  // (2^89, 2^-40)
-constexpr float kUnscale = 1099511627776.f;    // 2^40
-// 8 codes of a word as (c0,c4) (c1,c5) (c2,c6) (c3,c7), the order in which the nibble masks give them
-__device__ __forceinline__ void dequant8_q4(uint32_t w, uint32_t s_lo, uint32_t s_hi, uint32_t b2, uint32_t (&out)[4]) {
-    const uint32_t v = w >> 8;
-    out[0] = fma_bf2(w & 0x000f000fu, s_lo, b2);
-    out[1] = fma_bf2(w & 0x00f000f0u, s_hi, b2);
-    out[2] = fma_bf2(v & 0x000f000fu, s_lo, b2);
-    out[3] = fma_bf2(v & 0x00f000f0u, s_hi, b2);
-}
 
 // four consecutive features of a token
 template <int EPI>
@@ -214,11 +183,10 @@ __global__ void __launch_bounds__(kThreads, 2)
                     for (int i = 0; i < 2; i++) {
                         const uint4& wi = w[sp][i];
                         if (WK == 4) {
-                            dequant8_q4((&wi.x)[e8], s_lo[i], s_hi[i], b2[i], o[i]);
+                            scaled_q4_paired((&wi.x)[e8], s_lo[i], s_hi[i], b2[i], o[i]);
                         } else if (WK == 8) {
-#pragma unroll
-                            for (int j = 0; j < 4; j++)
-                                o[i][j] = fma_bf2(prmt((&wi.x)[(2 * e8 + j / 2) & 3], 0u, j & 1 ? 0x4342u : 0x4140u), s_lo[i], b2[i]);
+                            scaled_q8((&wi.x)[2 * e8 & 3], s_lo[i], b2[i], o[i][0], o[i][1]);
+                            scaled_q8((&wi.x)[(2 * e8 + 1) & 3], s_lo[i], b2[i], o[i][2], o[i][3]);
                         } else {
                             o[i][0] = wi.x, o[i][1] = wi.y, o[i][2] = wi.z, o[i][3] = wi.w;
                         }

@@ -44,6 +44,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "dequant.cuh"
 #include "kernels.h"
 
 namespace {
@@ -168,16 +169,6 @@ __device__ __forceinline__ uint32_t sub_bf2(uint32_t a, uint32_t b) {
     asm("sub.rn.bf16x2 %0, %1, %2;\n" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-__device__ __forceinline__ uint32_t fma_bf2(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.bf16x2 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
 // 32-byte read-only global load (32-byte aligned address) that leaves no copy in L1: every code is read once, and
 // keeping the lines out of L1 measured 2-6 % on every shape
 __device__ __forceinline__ void ldg256(const uint4* p, uint4& a, uint4& b) {
@@ -265,7 +256,9 @@ __device__ __forceinline__ Piece piece_at(int unit, int unit_end, int bpt, int b
     return pc;
 }
 
-template <int WK, int EPI>
+// With the table a weight costs 1.5 instructions (Q4) or 1 (Q8) instead of 2.4 and 3.5 (dequant.cuh): steps of the 8B Q4 model with 64
+// sequences 6.52 -> 6.27 ms, with 96 and a 512-token portion 13.56 -> 13.25, the 32B Q8 model's 512-token portion (8 layers) 8.25 -> 7.94.
+template <int WK, int EPI, bool TABLE>  // TABLE: scales and biases come as GemmParams::sbt, whose words may be scaled (dequant.cuh)
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_tc_pair_kernel(const GemmParams p, const PairPlan plan, const __grid_constant__ CUtensorMap map_x,
                         const __grid_constant__ CUtensorMap map_x_small, const __grid_constant__ CUtensorMap map_w) {
@@ -345,7 +338,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 const uint4* wq = reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(p.w) + (size_t)(row_ok ? gn : 0) * (K * WK / 32));
                 const uint16_t* sc_row = p.scales + (size_t)(row_ok ? gn : 0) * groups;
                 const uint16_t* bi_row = p.biases + (size_t)(row_ok ? gn : 0) * groups;
-                const uint32_t* sbt_col = p.sbt ? p.sbt + (row_ok ? gn : 0) : nullptr;
+                const uint32_t* sbt_col = TABLE ? p.sbt + (row_ok ? gn : 0) : nullptr;
                 constexpr int NQ = WK == 4 ? 2 : 4;  // 16-byte loads per 64 codes
                 // Codes, scale and bias of the next DEPTH slabs of this group wait in registers (DEPTH * GROUPS slabs
                 // ahead of the one being dequantised): the loads come from DRAM or a busy L2, and with a single slab
@@ -368,7 +361,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     // rows read one 128-byte line), two 2-byte loads that each touch 32 lines where it does not
                     if (!row_ok)
                         sb[d] = 0u;
-                    else if (sbt_col)
+                    else if (TABLE)
                         sb[d] = __ldg(sbt_col + (size_t)kb * N);
                     else
                         sb[d] = (uint32_t)__ldg(sc_row + kb) | ((uint32_t)__ldg(bi_row + kb) << 16);
@@ -397,7 +390,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         alive = false;
                         break;
                     }
-                    if (WK == 4) {
+                    if (TABLE) {
+                        const uint32_t b2 = mul_bf2(cbi * 0x10001u, 0x2b802b80u);
+                        if (WK == 4) {
+                            const uint32_t scales = mul_bf2(csc * 0x10001u, 0x6c006e00u);
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                uint32_t o[4];
+                                scaled_q4((&cd[i >> 2].x)[i & 3], scales, b2, o);
+                                sts128(sA + ((((uint32_t)i) ^ sw) << 4), o[0], o[1], o[2], o[3]);
+                            }
+                        } else {
+                            const uint32_t s2 = mul_bf2(csc * 0x10001u, 0x6e006e00u);
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                uint32_t o[4];
+                                scaled_q8((&cd[(i >> 1) & (NQ - 1)].x)[2 * i & 3], s2, b2, o[0], o[1]);
+                                scaled_q8((&cd[(i >> 1) & (NQ - 1)].x)[(2 * i + 1) & 3], s2, b2, o[2], o[3]);
+                                sts128(sA + ((((uint32_t)i) ^ sw) << 4), o[0], o[1], o[2], o[3]);
+                            }
+                        }
+                    } else if (WK == 4) {
                         const uint32_t s2 = csc * 0x10001u, b2 = cbi * 0x10001u;
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
@@ -496,7 +509,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     for (int i = 0; i < 32; i++) {
                         if (i >= left) break;
                         const int t = tg + i;
-                        const float a = __uint_as_float(v[i]);
+                        const float a = TABLE ? __uint_as_float(v[i]) * kUnscale : __uint_as_float(v[i]);
                         if (splits > 1) {
                             plan.partial[((size_t)pc.split * M + t) * N + f] = a;
                         } else if (EPI == EPI_F32) {
@@ -784,9 +797,9 @@ __global__ void sbt_build_kernel(const uint16_t* __restrict__ scales, const uint
     }
 }
 
-template <int WK, int EPI>
+template <int WK, int EPI, bool TABLE>
 int32_t launch_pair(b2_ctx* ctx, const GemmParams& p, int* err) {
-    B2_SMEM_ONCE(ctx, (gemm_tc_pair_kernel<WK, EPI>), SMEM_BYTES);
+    B2_SMEM_ONCE(ctx, (gemm_tc_pair_kernel<WK, EPI, TABLE>), SMEM_BYTES);
     PairPlan plan{};
     plan.block_tokens = 256;
     plan.blocks_per_tile = (p.M + plan.block_tokens - 1) / plan.block_tokens;
@@ -843,10 +856,10 @@ int32_t launch_pair(b2_ctx* ctx, const GemmParams& p, int* err) {
     cfg.numAttrs = 1;
     // with split K the pair kernel only writes partial sums: the residual variant's extra registers buy nothing there
     if (best > 1 && EPI == EPI_BF16_RESADD) {
-        B2_SMEM_ONCE(ctx, (gemm_tc_pair_kernel<WK, EPI_BF16>), SMEM_BYTES);
-        B2_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<WK, EPI_BF16>, p, plan, map_x, map_s, map_w));
+        B2_SMEM_ONCE(ctx, (gemm_tc_pair_kernel<WK, EPI_BF16, TABLE>), SMEM_BYTES);
+        B2_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<WK, EPI_BF16, TABLE>, p, plan, map_x, map_s, map_w));
     } else {
-        B2_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<WK, EPI>, p, plan, map_x, map_s, map_w));
+        B2_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<WK, EPI, TABLE>, p, plan, map_x, map_s, map_w));
     }
     B2_LAUNCHED(ctx);
     if (best > 1) {
@@ -864,14 +877,20 @@ int32_t launch_pair(b2_ctx* ctx, const GemmParams& p, int* err) {
     return B2_OK;
 }
 
-template <int WK>
-int32_t dispatch_pair(b2_ctx* ctx, const GemmParams& p, int* err) {
+template <int WK, bool TABLE>
+int32_t dispatch_epi(b2_ctx* ctx, const GemmParams& p, int* err) {
     switch (p.epilogue) {
-        case EPI_BF16: return launch_pair<WK, EPI_BF16>(ctx, p, err);
-        case EPI_BF16_RESADD: return launch_pair<WK, EPI_BF16_RESADD>(ctx, p, err);
-        case EPI_F32: return launch_pair<WK, EPI_F32>(ctx, p, err);
+        case EPI_BF16: return launch_pair<WK, EPI_BF16, TABLE>(ctx, p, err);
+        case EPI_BF16_RESADD: return launch_pair<WK, EPI_BF16_RESADD, TABLE>(ctx, p, err);
+        case EPI_F32: return launch_pair<WK, EPI_F32, TABLE>(ctx, p, err);
     }
     return b2_fail(B2_ERR_MSG, "gemm: bad epilogue");
+}
+template <int WK>
+int32_t dispatch_pair(b2_ctx* ctx, const GemmParams& p, int* err) {
+    if constexpr (WK != 0)
+        if (p.sbt) return dispatch_epi<WK, true>(ctx, p, err);
+    return dispatch_epi<WK, false>(ctx, p, err);
 }
 
 }  // namespace
