@@ -172,30 +172,31 @@ int32_t set_local_dims(b2_model* m, b2_tp_group* tp) {
 // The projection kernels take scale and bias of a tile's feature rows at one K group as consecutive words: a second
 // copy of both, transposed and interleaved, makes that one line for 32 rows instead of 64.  (Not counted in weight_bytes: it is a
 // derived layout, 1/9 of the packed 4-bit codes.)
-static int32_t build_sbt(b2_model* m, Proj& p) {
+static int32_t build_sbt(b2_model* m, Proj& p, int* wide_dev) {
     if (p.bits == 0 || p.sbt) return B2_OK;
     const int G = p.K / 64;
-    uint32_t* table = nullptr;
-    int usable = 0;
-    B2_CUDA(cudaMalloc((void**)&table, (size_t)p.N * G * 4));
-    const int32_t rc = b2_gemm_build_sbt(m->ctx, p.scales, p.biases, p.N, G, table, &usable);
-    if (rc != B2_OK || !usable) {
-        cudaFree(table);
-        return rc;
-    }
-    p.sbt = table;
-    m->allocs.push_back(table);
-    return B2_OK;
+    B2_CUDA(cudaMalloc((void**)&p.sbt, (size_t)p.N * G * 4));
+    m->allocs.push_back(p.sbt);
+    return b2_gemm_build_sbt(m->ctx, p.scales, p.biases, p.N, G, p.sbt, wide_dev);
 }
 
 int32_t finish_model(b2_model* m) {
-    for (auto& L : m->layers) {
-        B2_CHECK(build_sbt(m, L.qkv));
-        B2_CHECK(build_sbt(m, L.o));
-        B2_CHECK(build_sbt(m, L.gu));
-        B2_CHECK(build_sbt(m, L.down));
+    const size_t tables = 4 * m->layers.size();
+    std::vector<int> wide(tables, 0);  // tables whose words cannot be scaled
+    void* flags = nullptr;
+    if (tables) {
+        B2_CHECK(b2_ctx_scratch(m->ctx, tables * sizeof(int), &flags));
+        B2_CUDA(cudaMemsetAsync(flags, 0, tables * sizeof(int), m->ctx->stream));
     }
+    int* flag = (int*)flags;
+    for (auto& L : m->layers)
+        for (Proj* p : {&L.qkv, &L.o, &L.gu, &L.down}) B2_CHECK(build_sbt(m, *p, flag++));
+    if (tables) B2_CUDA(cudaMemcpyAsync(wide.data(), flags, tables * sizeof(int), cudaMemcpyDeviceToHost, m->ctx->stream));
     B2_CUDA(cudaStreamSynchronize(m->ctx->stream));
+    const int* found = wide.data();
+    for (auto& L : m->layers)
+        for (Proj* p : {&L.qkv, &L.o, &L.gu, &L.down})
+            if (*found++) p->sbt = nullptr;  // (its memory stays with the model's)
     m->inv_freq.resize(m->cfg.head_dim / 2);
     B2_CHECK(b2_rope_inv_freq(m->cfg.head_dim, m->cfg.rope_theta, m->cfg.rope_kind, m->cfg.rope_factor, m->cfg.rope_low_freq_factor,
                               m->cfg.rope_high_freq_factor, m->cfg.rope_original_context, m->inv_freq.data()));

@@ -895,17 +895,10 @@ int32_t dispatch_pair(b2_ctx* ctx, const GemmParams& p, int* err) {
 
 }  // namespace
 
-int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev, int* usable) {
-    void* wide = nullptr;
-    int found = 0;
-    B2_CHECK(b2_ctx_scratch(ctx, sizeof(int), &wide));
-    B2_CUDA(cudaMemsetAsync(wide, 0, sizeof(int), ctx->stream));
-    sbt_build_kernel<<<dim3((unsigned)((G + 31) / 32), (unsigned)((N + 31) / 32)), dim3(32, 8), 0, ctx->stream>>>(scales_dev, biases_dev, N, G, sbt_dev, (int*)wide);
+int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev, int* wide_dev) {
+    sbt_build_kernel<<<dim3((unsigned)((G + 31) / 32), (unsigned)((N + 31) / 32)), dim3(32, 8), 0, ctx->stream>>>(scales_dev, biases_dev, N, G, sbt_dev, wide_dev);
     B2_LAUNCHED(ctx);
     B2_CUDA(cudaGetLastError());
-    B2_CUDA(cudaMemcpyAsync(&found, wide, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    B2_CUDA(cudaStreamSynchronize(ctx->stream));
-    *usable = !found;
     return B2_OK;
 }
 

@@ -87,9 +87,10 @@ int32_t b2_gemm_ring_launch(b2_ctx* ctx, const GemmParams& p);
 // tcgen05 / TMEM path, CTA-pair form (gemm_tc.cu): taken by b2_gemm_launch when eligible.
 bool b2_gemm_tc_eligible(const GemmParams& p);
 int32_t b2_gemm_tc_launch(b2_ctx* ctx, const GemmParams& p);
-// Fills sbt (N * G words) from scales / biases [N, G] (see GemmParams::sbt) and waits for it.  *usable is 0 when a scale is 2^33 or
-// more in size, infinite or not a number: the kernels that take the table scale its words by powers of two (gemm_ring.cu).
-int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev, int* usable);
+// Fills sbt (N * G words) from scales / biases [N, G] (see GemmParams::sbt); enqueued on the context's stream.  *wide_dev becomes 1
+// when a scale is 2^33 or more in size, infinite or not a number: such a table must not be used, since the kernels that take it
+// scale its words by powers of two (dequant.cuh).
+int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev, int* wide_dev);
 
 // ---- elementwise / normalisation / embedding / sampling (fused_ops.cu) ---------------------------
 // out = rmsnorm(x) * w, one row per token; rows gathered through `row_idx` when non-null.
