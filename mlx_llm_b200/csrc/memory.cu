@@ -8,6 +8,8 @@
 // A sequence that starts in this step (nothing cached) starts from zero, whatever its slot held before.
 //
 // Everything that enters the recurrence besides the convolved (or plain) values is prepared and kept in f32.
+#include <type_traits>
+
 #include "elt.cuh"
 #include "memory.cuh"
 
@@ -382,11 +384,13 @@ __global__ void __launch_bounds__(256) memory_prep_kernel(const MemorySpec s, co
 // state answers to its key and to its query -- are taken together: S_new^T q = S^T q + u (k . q).  With a bonus the read-out
 // comes before the decay, and the keys in k . q are weighted by it.
 constexpr int SC_P = 16;
-template <typename T, int K4, bool BONUS>
+// SC_T tokens at a time: with a buffer for sixteen only nine blocks fit an SM, and the 2048 blocks of a step of single tokens (16
+// sequences, 16 heads of 128 x 128) take two rounds; such steps take one token at a time (12.3 -> 11.1 us).
+template <typename T, int K4, bool BONUS, int SC_T>
 __global__ void __launch_bounds__(128) memory_scan_kernel(const MemorySpec s, const MemoryParams p) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     pdl_wait();
-    constexpr int NP = K4 * 32, SC_T = K4 <= 4 ? 16 : 8;
+    constexpr int NP = K4 * 32;
     __shared__ __align__(16) float Ks[SC_T][NP], Qs[SC_T][NP], Gs[SC_T][NP];
     __shared__ float xs[SC_T][SC_P], kq[SC_T], bs[SC_T];
     const int h = blockIdx.y, b = blockIdx.z, p0 = blockIdx.x * SC_P, kh = h / (s.heads / s.kv_heads);
@@ -633,9 +637,15 @@ int32_t launch_memory(b2_ctx* ctx, const MemorySpec& s, const MemoryParams& p) {
     if (p.n_chunks > 0) B2_CHECK(b2_memory_chunk_launch(ctx, s, p));
     if (p.n_chunks == 0 || p.B > 1) {
         const int k4 = (s.dim + 31) / 32;
-        auto k = s.bonus ? (k4 <= 1 ? memory_scan_kernel<T, 1, true> : k4 <= 2 ? memory_scan_kernel<T, 2, true> : k4 <= 4 ? memory_scan_kernel<T, 4, true> : memory_scan_kernel<T, 8, true>)
-                         : (k4 <= 1 ? memory_scan_kernel<T, 1, false> : k4 <= 2 ? memory_scan_kernel<T, 2, false> : k4 <= 4 ? memory_scan_kernel<T, 4, false> : memory_scan_kernel<T, 8, false>);
-        B2_CUDA(b2_launch_pdl(ctx->pdl_consumers, k, dim3((s.vdim + SC_P - 1) / SC_P, s.heads, p.B), dim3(128), 0, ctx->stream, s, p));
+        auto go = [&](auto single) -> int32_t {
+            constexpr bool ONE = decltype(single)::value;
+            constexpr int FEW = ONE ? 1 : 16, MANY = ONE ? 1 : 8;
+            auto k = s.bonus ? (k4 <= 1 ? memory_scan_kernel<T, 1, true, FEW> : k4 <= 2 ? memory_scan_kernel<T, 2, true, FEW> : k4 <= 4 ? memory_scan_kernel<T, 4, true, FEW> : memory_scan_kernel<T, 8, true, MANY>)
+                             : (k4 <= 1 ? memory_scan_kernel<T, 1, false, FEW> : k4 <= 2 ? memory_scan_kernel<T, 2, false, FEW> : k4 <= 4 ? memory_scan_kernel<T, 4, false, FEW> : memory_scan_kernel<T, 8, false, MANY>);
+            B2_CUDA(b2_launch_pdl(ctx->pdl_consumers, k, dim3((s.vdim + SC_P - 1) / SC_P, s.heads, p.B), dim3(128), 0, ctx->stream, s, p));
+            return B2_OK;
+        };
+        B2_CHECK(p.T == p.B ? go(std::true_type{}) : go(std::false_type{}));
         B2_LAUNCHED(ctx);
     }
     return B2_OK;
