@@ -174,11 +174,17 @@ __global__ void post_norm_kernel(const PostNormParams p) {
 template <typename T, int NV>
 __global__ void __launch_bounds__(NV <= 1 ? 1024 : 512) post_norm_rows_kernel(const PostNormParams p) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    pdl_wait();
     extern __shared__ float part[];  // [width / 128] sums of squares
     const size_t r = blockIdx.x;
     const int size = p.width / p.groups, per = size / 128, lane = threadIdx.x & 31;
     float y[NV][4], x[NV][4], w[NV][4];
+#pragma unroll
+    for (int k = 0; k < NV; k++) {  // (the weights before the wait: nothing earlier writes them; one row 4.7 -> 4.5 us)
+        const int i = (threadIdx.x + k * blockDim.x) * 4;
+        if (i < p.width) Elt<float>::ld4(p.w + i, w[k]);
+    }
+    const float own = p.avg ? p.avg[p.depth] : 1.f;
+    pdl_wait();
     const float* yr = p.y + (p.y_rows ? (size_t)p.y_rows[r] : r) * p.ldy;
 #pragma unroll
     for (int k = 0; k < NV; k++) {
@@ -191,7 +197,6 @@ __global__ void __launch_bounds__(NV <= 1 ? 1024 : 512) post_norm_rows_kernel(co
         x[k][0] = x[k][1] = x[k][2] = x[k][3] = 0.f;
         if (i >= p.width) continue;
         if (p.x) Elt<float>::ld4(p.x + r * p.ldx + i, x[k]);
-        Elt<float>::ld4(p.w + i, w[k]);
     }
     float past[NV][4];
 #pragma unroll
@@ -218,7 +223,6 @@ __global__ void __launch_bounds__(NV <= 1 ? 1024 : 512) post_norm_rows_kernel(co
         if (lane == 0) part[i / 128] = ss;
     }
     __syncthreads();
-    const float own = p.avg ? p.avg[p.depth] : 1.f;
     T* o = p.out ? reinterpret_cast<T*>(p.out) + r * p.ldo : nullptr;
 #pragma unroll
     for (int k = 0; k < NV; k++) {
@@ -258,6 +262,14 @@ __global__ void token_gate_kernel(const TokenGateParams p) {
     }
 }
 
+// The norm's weights of a thread's first eight columns: loaded before the wait for the kernel in front, which does not write them
+// (streams' step of 8 tokens 5.2 -> 4.7 us, of 2076 49.8 -> 47.9).
+__device__ __forceinline__ void early_weights(const float* w, int width, float (&v)[8]) {
+    const int i = threadIdx.x * 8;
+    const bool some = w && width % 8 == 0 && i < width;
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = some ? w[i + j] : 0.f;
+}
 // x += y (one row, or the sum of several), then RMS norm, one block per row.  The row is kept in shared memory between
 // the two passes.
 template <typename T>
@@ -337,6 +349,8 @@ __global__ void __launch_bounds__(NS <= 4 ? 1024 : 512) stream_norm_kernel(const
             from[b] = b < n ? (p.from ? p.from[b] : 1.f) : 0.f;
         }
     }
+    float early[8];
+    early_weights(p.w, p.width, early);
     pdl_wait();
     const int r = blockIdx.x, t = p.row_idx ? p.row_idx[r] : r;
     float* xt = p.x + (size_t)t * n * p.ldx;
@@ -430,7 +444,7 @@ __global__ void __launch_bounds__(NS <= 4 ? 1024 : 512) stream_norm_kernel(const
         for (int i = threadIdx.x * 8; i < p.ldo; i += blockDim.x * 8) {
             float v[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = i < p.width ? row[i + j] * inv * p.w[i + j] * p.out_scale : 0.f;
+            for (int j = 0; j < 8; j++) v[j] = i < p.width ? row[i + j] * inv * (i == (int)threadIdx.x * 8 ? early[j] : p.w[i + j]) * p.out_scale : 0.f;
             Elt<T>::st8(o + i, v);
         }
     } else {
