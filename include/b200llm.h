@@ -169,6 +169,14 @@ int32_t b2_qmm_host(b2_ctx* ctx, const uint16_t* x_host, const uint32_t* packed_
 int32_t b2_linear(b2_ctx* ctx, const uint16_t* x_dev, const uint16_t* w_dev, int32_t m, int32_t out_dim, int32_t in_dim,
                   uint16_t* y_bf16_dev, float* y_f32_dev);
 
+/* One projection on the path that a model's layers take, for parity tests: W dense (bits 0) or quantized and then with the table of
+ * scales and biases that a model builds at load (built anew by every call, which waits for it).  One output of the three: y = x W^T
+ * as bf16 or f32, or h = bf16(h + bf16(x W^T)) in place.  route_host (nullable, 4 values): the kernel (0 tiles, 1 weight streaming,
+ * 2 weight ring, 3 CTA pairs), 1 if it reads the table, its K ranges, the blocks of a cluster that share them (ring). */
+int32_t b2_projection(b2_ctx* ctx, const uint16_t* x_dev, const void* w_dev, const uint16_t* scales_dev, const uint16_t* biases_dev,
+                      int32_t m, int32_t out_dim, int32_t in_dim, int32_t bits, uint16_t* y_bf16_dev, float* y_f32_dev, uint16_t* h_dev,
+                      int32_t* route_host);
+
 /* ---- fused leaves --------------------------------------------------------------------------- */
 /* rms_norm (src/primitives/nn.rs:35-37): out = bf16(x / rms(x) * w), rows of `dim`. */
 int32_t b2_rms_norm(b2_ctx* ctx, const uint16_t* x_dev, const uint16_t* w_dev, float eps, int32_t rows, int32_t dim,

@@ -144,6 +144,54 @@ int32_t b2_linear(b2_ctx* ctx, const uint16_t* x_dev, const uint16_t* w_dev, int
     return gemm_both(ctx, p, y_bf16_dev, y_f32_dev);
 }
 
+// One projection on the path that a model's layers take: quantized weights come with their table of scales and biases.
+int32_t b2_projection(b2_ctx* ctx, const uint16_t* x_dev, const void* w_dev, const uint16_t* scales_dev, const uint16_t* biases_dev, int32_t m, int32_t out_dim,
+                      int32_t in_dim, int32_t bits, uint16_t* y_bf16_dev, float* y_f32_dev, uint16_t* h_dev, int32_t* route_host) {
+    B2_REQUIRE(ctx && x_dev && w_dev && (bits == 0 || (scales_dev && biases_dev)), B2_ERR_MSG, "b2_projection: null argument");
+    B2_REQUIRE(bits == 0 || bits == 4 || bits == 8, B2_ERR_UNSUPPORTED, "b2_projection: bits must be 0, 4 or 8");
+    B2_REQUIRE(m >= 0 && out_dim > 0 && in_dim > 0 && (bits == 0 || in_dim % 64 == 0), B2_ERR_MSG, "b2_projection: bad shape");
+    B2_REQUIRE((y_bf16_dev != nullptr) + (y_f32_dev != nullptr) + (h_dev != nullptr) == 1, B2_ERR_MSG, "b2_projection: one output buffer is wanted");
+    GemmParams p{};
+    if (bits) {
+        const size_t words = (size_t)out_dim * (in_dim / 64);
+        void* scratch = nullptr;
+        int wide = 0;
+        B2_CHECK(b2_ctx_scratch(ctx, (words + 1) * 4, &scratch));
+        uint32_t* table = (uint32_t*)scratch;
+        B2_CUDA(cudaMemsetAsync(table + words, 0, 4, ctx->stream));
+        B2_CHECK(b2_gemm_build_sbt(ctx, scales_dev, biases_dev, out_dim, in_dim / 64, table, (int*)(table + words)));
+        B2_CUDA(cudaMemcpyAsync(&wide, table + words, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        B2_CUDA(cudaStreamSynchronize(ctx->stream));
+        if (!wide) p.sbt = table;
+    }
+    p.x = x_dev;
+    p.w = w_dev;
+    p.scales = scales_dev;
+    p.biases = biases_dev;
+    p.bits = bits;
+    p.group = 64;
+    p.M = m;
+    p.N = out_dim;
+    p.K = in_dim;
+    p.ldx = in_dim;
+    p.ldo = out_dim;
+    p.ldres = out_dim;
+    p.epilogue = h_dev ? EPI_BF16_RESADD : y_f32_dev ? EPI_F32 : EPI_BF16;
+    p.out = h_dev ? h_dev : y_bf16_dev;
+    p.res = h_dev;
+    p.out_f32 = y_f32_dev;
+    if (route_host) {
+        const GemmKernel kernel = b2_gemm_pick(ctx, p);
+        int cluster = 0;
+        if (kernel == GEMM_RING) B2_CHECK(b2_gemm_ring_launch(ctx, p, &cluster));
+        route_host[0] = kernel;
+        route_host[1] = p.sbt != nullptr;
+        route_host[2] = kernel == GEMM_RING || kernel == GEMM_STREAM ? b2_gemm_stream_ranges(ctx, p.N, p.K).ranges : 1;
+        route_host[3] = cluster;
+    }
+    return b2_gemm_launch(ctx, p);
+}
+
 int32_t b2_rms_norm(b2_ctx* ctx, const uint16_t* x_dev, const uint16_t* w_dev, float eps, int32_t rows, int32_t dim, uint16_t* out_dev) {
     B2_REQUIRE(ctx && x_dev && w_dev && out_dev, B2_ERR_MSG, "b2_rms_norm: null argument");
     return b2_rms_norm_launch(ctx, x_dev, w_dev, eps, rows, dim, dim, nullptr, out_dev);

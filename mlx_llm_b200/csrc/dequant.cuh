@@ -1,10 +1,10 @@
 // Group-quantized codes to bf16 weights without a conversion.
 //
 // An unsigned byte c in the low bits of a bf16, with nothing above it, IS the number c 2^-133 (up to 127 a subnormal, from 128 on the
-// exponent's lowest bit takes over where they end).  One fma with scale 2^93 and bias 2^-40 then gives bf16(c scale + bias) 2^-40 with
-// the one rounding that the format asks for; the f32 sums are scaled back at the end.  A nibble in bits 4-7 counts 2^4 times as much.
-// (A Q8 weight that an f32 fma and a second rounding to bf16 give can differ in its last bit where the scale is 2^14 or more below the
-// bias, a handful in a billion.)  Exact for scales below 2^33 and weights above 2^-86; a matrix with a larger scale gets no table (b2_gemm_build_sbt) and stays with
+// exponent's lowest bit takes over where they end).  One fma with scale 2^93 and bias 2^-40 then gives bf16(c scale + bias) 2^-40;
+// the f32 sums are scaled back at the end.  A nibble in bits 4-7 counts 2^4 times as much.  Q4 weights are rounded once in every
+// projection kernel; Q8 weights are an f32 fma, then rounded to bf16 (b2_dequantize, the kernels without a table), and so they are here.
+// Exact for scales below 2^33 and weights above 2^-86; a matrix with a larger scale gets no table (b2_gemm_build_sbt) and stays with
 // the kernels that mask into 128 + c and subtract.
 #pragma once
 #include "common.cuh"
@@ -43,8 +43,24 @@ __device__ __forceinline__ void scaled_q4_paired(uint32_t w, uint32_t s_lo, uint
     out[2] = fma_bf2(v & 0x000f000fu, s_lo, b2);
     out[3] = fma_bf2(v & 0x00f000f0u, s_hi, b2);
 }
-// 4 Q8 codes
-__device__ __forceinline__ void scaled_q8(uint32_t w, uint32_t s2, uint32_t b2, uint32_t& lo, uint32_t& hi) {
+// 4 Q8 codes: a byte two bytes up is the same number in f32, and two of them are one fma
+__device__ __forceinline__ void scaled_q8(uint32_t w, float scale, float bias, uint32_t& lo, uint32_t& hi) {
+    auto pair = [&](uint32_t c0, uint32_t c1) {
+        uint64_t r;
+        asm("{\n.reg .b64 c, s, b;\nmov.b64 c, {%1, %2};\nmov.b64 s, {%3, %3};\nmov.b64 b, {%4, %4};\nfma.rn.f32x2 %0, c, s, b;\n}\n"
+            : "=l"(r)
+            : "r"(c0), "r"(c1), "f"(scale), "f"(bias));
+        return pack_bf2(__uint_as_float((uint32_t)r), __uint_as_float((uint32_t)(r >> 32)));
+    };
+    lo = pair(prmt(w, 0u, 0x4044u), prmt(w, 0u, 0x4144u));
+    hi = pair(prmt(w, 0u, 0x4244u), prmt(w, 0u, 0x4344u));
+}
+// The same weights by half the instructions, where one_rounding() holds.
+__device__ __forceinline__ void scaled_q8_once(uint32_t w, uint32_t s2, uint32_t b2, uint32_t& lo, uint32_t& hi) {
     lo = fma_bf2(prmt(w, 0u, 0x4140u), s2, b2);
     hi = fma_bf2(prmt(w, 0u, 0x4342u), s2, b2);
 }
+// One fma in bf16 gives the bits of the two roundings unless the first drops a bias so small that code scale alone is a tie of the
+// second: never where the scale's exponent is at most 15 above the bias's (all mantissas, codes and signs tried; from 16 on 1 weight
+// in 70 000 differs, and more).  For a table word, the difference of its exponents times 2^23, less at most 2^15.
+__device__ __forceinline__ bool one_rounding(uint32_t sb) { return (int)((sb & 0x7f807f80u) * 0xffffu) < (16 << 23) - (1 << 15); }

@@ -22,6 +22,7 @@
 // 67.1 -> 35.7, 9.2 -> 6.0, 185 -> 170.  With 17 to 32 tokens on Q4 the activations leave the ring too few stages, and the other
 // kernel is faster; on Q8 and bf16 it is not (32 tokens: 51200 x 5120 Q8 128 -> 79, 28672 x 4096 bf16 62 -> 55).
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "dequant.cuh"
@@ -162,17 +163,24 @@ __global__ void __launch_bounds__(kThreads, 2)
             for (int sp = 0; sp < 2; sp++)
 #pragma unroll
                 for (int i = 0; i < 2; i++) w[sp][i] = lds128(ring + s * kTileBytes + (row + i * 8) * kRowBytes + (((4 * sp + t) ^ rg) << 4));
+            uint32_t sb[2][2];
+            bool all_once = true;
+            if (WK)
 #pragma unroll
-            for (int sp = 0; sp < 2; sp++) {
+                for (int j = 0; j < 4; j++) {
+                    const int sp = j >> 1, i = j & 1;
+                    sb[sp][i] = lds32(sbring + s * R::SB_BYTES + (WK == 4 ? 2 * sp + (t >> 1) : sp) * kGroupStride + (row + i * 8) * 4);
+                    if (WK == 8) all_once = all_once && one_rounding(sb[sp][i]);
+                }
+            auto half = [&](int sp, auto once) {
                 uint32_t s_lo[2], s_hi[2], b2[2];
                 if (WK)
 #pragma unroll
                     for (int i = 0; i < 2; i++) {
-                        const uint32_t sb = lds32(sbring + s * R::SB_BYTES + (WK == 4 ? 2 * sp + (t >> 1) : sp) * kGroupStride + (row + i * 8) * 4);
-                        const uint32_t lo = mul_bf2(sb, kByteUnit);
+                        const uint32_t lo = mul_bf2(sb[sp][i], kByteUnit);
                         s_lo[i] = prmt(lo, lo, 0x1010u), b2[i] = prmt(lo, lo, 0x3232u);
                         if (WK == 4) {
-                            const uint32_t hi = mul_bf2(sb, kNibbleUnit);
+                            const uint32_t hi = mul_bf2(sb[sp][i], kNibbleUnit);
                             s_hi[i] = prmt(hi, hi, 0x1010u);
                         }
                     }
@@ -185,8 +193,14 @@ __global__ void __launch_bounds__(kThreads, 2)
                         if (WK == 4) {
                             scaled_q4_paired((&wi.x)[e8], s_lo[i], s_hi[i], b2[i], o[i]);
                         } else if (WK == 8) {
-                            scaled_q8((&wi.x)[2 * e8 & 3], s_lo[i], b2[i], o[i][0], o[i][1]);
-                            scaled_q8((&wi.x)[(2 * e8 + 1) & 3], s_lo[i], b2[i], o[i][2], o[i][3]);
+#pragma unroll
+                            for (int j = 0; j < 2; j++) {
+                                const uint32_t codes = (&wi.x)[(2 * e8 + j) & 3];
+                                if (decltype(once)::value)
+                                    scaled_q8_once(codes, s_lo[i], b2[i], o[i][2 * j], o[i][2 * j + 1]);
+                                else
+                                    scaled_q8(codes, bflo(s_lo[i]), bflo(b2[i]), o[i][2 * j], o[i][2 * j + 1]);
+                            }
                         } else {
                             o[i][0] = wi.x, o[i][1] = wi.y, o[i][2] = wi.z, o[i][3] = wi.w;
                         }
@@ -208,6 +222,14 @@ __global__ void __launch_bounds__(kThreads, 2)
                         }
                     }
                 }
+            };
+            // (a choice for the whole stage: inside the loops it cost 7 %, the f32 fma throughout 10 %, of a step of 6 sequences)
+            if (WK != 8 || __all_sync(0xffffffffu, all_once)) {
+                half(0, std::true_type{});
+                half(1, std::true_type{});
+            } else {
+                half(0, std::false_type{});
+                half(1, std::false_type{});
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty(s));
@@ -304,7 +326,7 @@ int ring_splits(b2_ctx* ctx, int tiles, int ranges, int range_stages) {
 }
 
 template <int WK, int NT, int EPI>
-int32_t launch_ring(b2_ctx* ctx, const GemmParams& p) {
+int32_t launch_ring(b2_ctx* ctx, const GemmParams& p, int* cluster) {
     using R = Ring<WK, NT>;
     B2_SMEM_ONCE(ctx, (gemm_ring_kernel<WK, NT, EPI>), R::SMEM);
     const int tiles = p.N / kRows;
@@ -312,6 +334,10 @@ int32_t launch_ring(b2_ctx* ctx, const GemmParams& p) {
     const int range_stages = cut.k_per_range / R::KS;
     const int splits = ring_splits<WK, NT, EPI>(ctx, tiles, cut.ranges, range_stages);
     B2_REQUIRE(splits > 0, B2_ERR_MSG, "gemm: no split of K for the ring kernel");
+    if (cluster) {
+        *cluster = splits;
+        return B2_OK;
+    }
     EncodeTiledFn encode = encode_fn();
     B2_REQUIRE(encode != nullptr, B2_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     CUtensorMap map;
@@ -342,20 +368,20 @@ int32_t launch_ring(b2_ctx* ctx, const GemmParams& p) {
 }
 
 template <int WK, int NT>
-int32_t dispatch_epi(b2_ctx* ctx, const GemmParams& p) {
+int32_t dispatch_epi(b2_ctx* ctx, const GemmParams& p, int* cluster) {
     switch (p.epilogue) {
-        case EPI_BF16: return launch_ring<WK, NT, EPI_BF16>(ctx, p);
-        case EPI_BF16_RESADD: return launch_ring<WK, NT, EPI_BF16_RESADD>(ctx, p);
-        case EPI_F32: return launch_ring<WK, NT, EPI_F32>(ctx, p);
+        case EPI_BF16: return launch_ring<WK, NT, EPI_BF16>(ctx, p, cluster);
+        case EPI_BF16_RESADD: return launch_ring<WK, NT, EPI_BF16_RESADD>(ctx, p, cluster);
+        case EPI_F32: return launch_ring<WK, NT, EPI_F32>(ctx, p, cluster);
     }
     return b2_fail(B2_ERR_MSG, "gemm: bad epilogue");
 }
 
 template <int WK>
-int32_t dispatch_nt(b2_ctx* ctx, const GemmParams& p) {
-    if (p.M <= 8) return dispatch_epi<WK, 1>(ctx, p);
-    if (p.M <= 16) return dispatch_epi<WK, 2>(ctx, p);
-    if constexpr (WK != 4) return dispatch_epi<WK, 4>(ctx, p);
+int32_t dispatch_nt(b2_ctx* ctx, const GemmParams& p, int* cluster) {
+    if (p.M <= 8) return dispatch_epi<WK, 1>(ctx, p, cluster);
+    if (p.M <= 16) return dispatch_epi<WK, 2>(ctx, p, cluster);
+    if constexpr (WK != 4) return dispatch_epi<WK, 4>(ctx, p, cluster);
     return b2_fail(B2_ERR_MSG, "gemm: too many tokens for the ring kernel");
 }
 
@@ -376,8 +402,8 @@ bool b2_gemm_ring_eligible(b2_ctx* ctx, const GemmParams& p) {
     return (cut.ranges + 7) / 8 <= 1 + (p.M <= 8 ? Ring<0, 1>::kSlots : Ring<0, 2>::kSlots);
 }
 
-int32_t b2_gemm_ring_launch(b2_ctx* ctx, const GemmParams& p) {
-    if (p.bits == 0) return dispatch_nt<0>(ctx, p);
-    if (p.bits == 4) return dispatch_nt<4>(ctx, p);
-    return dispatch_nt<8>(ctx, p);
+int32_t b2_gemm_ring_launch(b2_ctx* ctx, const GemmParams& p, int* cluster) {
+    if (p.bits == 0) return dispatch_nt<0>(ctx, p, cluster);
+    if (p.bits == 4) return dispatch_nt<4>(ctx, p, cluster);
+    return dispatch_nt<8>(ctx, p, cluster);
 }

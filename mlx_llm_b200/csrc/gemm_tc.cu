@@ -256,7 +256,7 @@ __device__ __forceinline__ Piece piece_at(int unit, int unit_end, int bpt, int b
     return pc;
 }
 
-// With the table a weight costs 1.5 instructions (Q4) or 1 (Q8) instead of 2.4 and 3.5 (dequant.cuh): steps of the 8B Q4 model with 64
+// With the table a weight costs 1.5 instructions (Q4) or 2 (Q8) instead of 2.4 and 3.5 (dequant.cuh): steps of the 8B Q4 model with 64
 // sequences 6.52 -> 6.27 ms, with 96 and a 512-token portion 13.56 -> 13.25, the 32B Q8 model's 512-token portion (8 layers) 8.25 -> 7.94.
 template <int WK, int EPI, bool TABLE>  // TABLE: scales and biases come as GemmParams::sbt, whose words may be scaled (dequant.cuh)
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
@@ -401,12 +401,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                                 sts128(sA + ((((uint32_t)i) ^ sw) << 4), o[0], o[1], o[2], o[3]);
                             }
                         } else {
-                            const uint32_t s2 = mul_bf2(csc * 0x10001u, 0x6e006e00u);
+                            const float sf = bflo(mul_bf2(csc, 0x6e00u)), bf = bflo(b2);
 #pragma unroll
                             for (int i = 0; i < 8; i++) {
                                 uint32_t o[4];
-                                scaled_q8((&cd[(i >> 1) & (NQ - 1)].x)[2 * i & 3], s2, b2, o[0], o[1]);
-                                scaled_q8((&cd[(i >> 1) & (NQ - 1)].x)[(2 * i + 1) & 3], s2, b2, o[2], o[3]);
+                                scaled_q8((&cd[(i >> 1) & (NQ - 1)].x)[2 * i & 3], sf, bf, o[0], o[1]);
+                                scaled_q8((&cd[(i >> 1) & (NQ - 1)].x)[(2 * i + 1) & 3], sf, bf, o[2], o[3]);
                                 sts128(sA + ((((uint32_t)i) ^ sw) << 4), o[0], o[1], o[2], o[3]);
                             }
                         }

@@ -72,6 +72,8 @@ __device__ __forceinline__ float* gemm_f32_dst(const GemmParams& p, int t, int f
 }
 #endif
 int32_t b2_gemm_launch(b2_ctx* ctx, const GemmParams& p);
+enum GemmKernel { GEMM_TILE = 0, GEMM_STREAM = 1, GEMM_RING = 2, GEMM_PAIR = 3 };
+GemmKernel b2_gemm_pick(b2_ctx* ctx, const GemmParams& p);  // what b2_gemm_launch runs
 // weight-streaming kernel for up to 64 tokens (gemm_stream.cu): taken by b2_gemm_launch when eligible.
 bool b2_gemm_stream_eligible(const GemmParams& p);
 int32_t b2_gemm_stream_launch(b2_ctx* ctx, const GemmParams& p);
@@ -83,7 +85,8 @@ struct RangePlan {
 RangePlan b2_gemm_stream_ranges(b2_ctx* ctx, int N, int K);
 // up to 32 tokens (Q4: 16), for weights that come with a transposed table of scales and biases, or are dense (gemm_ring.cu)
 bool b2_gemm_ring_eligible(b2_ctx* ctx, const GemmParams& p);
-int32_t b2_gemm_ring_launch(b2_ctx* ctx, const GemmParams& p);
+// `cluster` non-null: no launch, *cluster becomes the number of blocks that would share a row tile's ranges.
+int32_t b2_gemm_ring_launch(b2_ctx* ctx, const GemmParams& p, int* cluster = nullptr);
 // tcgen05 / TMEM path, CTA-pair form (gemm_tc.cu): taken by b2_gemm_launch when eligible.
 bool b2_gemm_tc_eligible(const GemmParams& p);
 int32_t b2_gemm_tc_launch(b2_ctx* ctx, const GemmParams& p);

@@ -62,6 +62,14 @@ def linear(ctx, x, w, m, out_dim, in_dim, y_bf16=None, y_f32=None):
     check(load().b2_linear(ctx.h, ptr(x), ptr(w), int(m), int(out_dim), int(in_dim), ptr(y_bf16), ptr(y_f32)))
 
 
+def projection(ctx, x, w, scales, biases, m, out_dim, in_dim, bits, y_bf16=None, y_f32=None, h=None):
+    """One projection as a model's layers run it; returns (kernel, table used, K ranges, blocks per cluster)."""
+    route = (C.c_int32 * 4)()
+    check(load().b2_projection(ctx.h, ptr(x), ptr(w), ptr(scales), ptr(biases), int(m), int(out_dim), int(in_dim), int(bits), ptr(y_bf16),
+                               ptr(y_f32), ptr(h), route))
+    return tuple(route)
+
+
 def rms_norm(ctx, x, w, eps, rows, dim, out):
     check(load().b2_rms_norm(ctx.h, ptr(x), ptr(w), C.c_float(eps), int(rows), int(dim), ptr(out)))
 

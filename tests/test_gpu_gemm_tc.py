@@ -149,3 +149,49 @@ def test_ring_gemm_quantized_in_a_model(env, bits, batch):
     ctx, K, orc, _lib = env
     cfg = dict(LLAMA_CUT, layers=1, hidden=512, heads=4, kv_heads=1, inter=2816, vocab=1024, quant_bits=bits)
     run_schedule((ctx, engine, K, orc), cfg, [[(i, 2 + i % 3) for i in range(batch)], [(i, 1) for i in range(batch)]])
+
+
+def double_rounded(codes, scales, biases):
+    """bf16(f32(code scale + bias)) and bf16(code scale + bias) as bits; [n, k] codes, [n, k / 64] scales and biases."""
+    exact = codes.astype(np.float64) * np.repeat(H.bf16_to_f32_np(scales), 64, 1) + np.repeat(H.bf16_to_f32_np(biases), 64, 1)
+    twice = H.f32_to_bf16_np(exact.astype(np.float32))
+    # (the 52 bits of a double hold every sum here; odd behind the 16 bits of f32 that a bf16 drops: one rounding from there)
+    word = exact.astype(np.float32).view(np.uint32)
+    low = exact.astype(np.float32).astype(np.float64)
+    toward_zero = word - ((np.abs(low) > np.abs(exact)) & (word & 0x7fffffff > 0)).astype(np.uint32)
+    sticky = toward_zero | (low != exact).astype(np.uint32)
+    return twice, H.f32_to_bf16_np(sticky.view(np.float32))
+
+
+@pytest.mark.parametrize("m,kernel", [(8, 2), (16, 2), (32, 2), (512, 3)])
+def test_q8_weights_are_rounded_as_dequantize_does(env, m, kernel):
+    """Both kernels that read the table of scales and biases make the weights of b2_dequantize bit for bit, also where a bias far below
+    its scale decides a tie: an identity matrix as activations reads the weights out."""
+    ctx, K, orc, _lib = env
+    n, k = 256, 512
+    rng = np.random.default_rng(m)
+    codes = rng.integers(0, 256, (n, k), dtype=np.uint8)
+    mantissa = lambda: rng.integers(0, 128, (n, k // 64)) | rng.integers(0, 2, (n, k // 64)) << 15
+    down = rng.integers(-20, 28, (n, k // 64))  # bits that the bias lies below the scale
+    down[: n // 2] = np.clip(down[: n // 2], -20, 15)  # (row tiles without and with groups that are rounded twice)
+    scales = (mantissa() | 116 << 7).astype(np.uint16)
+    biases = (mantissa() | (116 - down) << 7).astype(np.uint16)
+    biases[3::7, 1] = 0
+    want, once = double_rounded(codes, scales, biases)
+    assert (want != once)[n // 2:].sum() > 20 and (want == once)[: n // 2].all()
+    packed = codes.view(np.uint32)
+    plain = ctx.empty((n, k), np.uint16)
+    dp, ds, db = ctx.buf(packed), ctx.buf(scales), ctx.buf(biases)
+    K.dequantize(ctx, dp, ds, db, n, k, 8, plain)
+    got = np.empty((n, k), np.uint16)
+    for at in range(0, k, m):
+        x = np.zeros((m, k), np.uint16)
+        x[np.arange(m), at + np.arange(m)] = 0x3f80
+        y = ctx.empty((m, n), np.uint16)
+        route = K.projection(ctx, ctx.buf(x), dp, ds, db, m, n, k, 8, y_bf16=y)
+        assert route[:2] == (kernel, 1)
+        ctx.sync()
+        got[:, at:at + m] = y.download().T
+    zero = (got & 0x7fff == 0) & (want & 0x7fff == 0)
+    assert ((got == want) | zero).all()
+    assert ((plain.download() == want) | zero).all()
