@@ -75,6 +75,7 @@ int32_t b2_qmm(b2_ctx* ctx, const uint16_t* x_dev, const uint32_t* packed_dev, c
     GemmParams p{};
     p.x = x_dev;
     p.w = packed_dev;
+    p.w_settled = true;
     p.scales = scales_dev;
     p.biases = biases_dev;
     p.bits = bits;
@@ -95,6 +96,7 @@ int32_t b2_qmm_residual(b2_ctx* ctx, const uint16_t* x_dev, const uint32_t* pack
     GemmParams p{};
     p.x = x_dev;
     p.w = packed_dev;
+    p.w_settled = true;
     p.scales = scales_dev;
     p.biases = biases_dev;
     p.bits = bits;
@@ -166,6 +168,7 @@ int32_t b2_projection(b2_ctx* ctx, const uint16_t* x_dev, const void* w_dev, con
     }
     p.x = x_dev;
     p.w = w_dev;
+    p.w_settled = bits != 0;
     p.scales = scales_dev;
     p.biases = biases_dev;
     p.bits = bits;

@@ -877,6 +877,7 @@ int32_t linear(b2_model* m, const Proj& p, const void* x, int ldx, int M, int ro
     GemmParams g{};
     g.x = (const uint16_t*)x;
     g.w = p.w;
+    g.w_settled = true;
     g.group = 64;
     g.M = M;
     g.N = p.N;

@@ -15,7 +15,7 @@
 //   * K is cut into the other kernel's ranges, each summed in K order by one warp, and the ranges are added in order: the results are
 //     that kernel's bits.  The blocks of a cluster share a row tile's ranges and add them up through distributed shared memory, where
 //     that kernel writes partial sums to global memory and lets the block that counts in last read them back.
-// The weights do not depend on the kernel before this one: the ring is filled with them before the wait for that kernel.
+// The weights of a model do not depend on the kernel before this one: the ring is filled with them before the wait for that kernel.
 // One token, us a call among others of its kind, register-streaming kernel -> this one (bytes at the copy rate): 28672 x 4096 Q4
 // 28.8 -> 22.7 (10.2), 4096 x 14336 Q4 17.6 -> 14.7 (5.1), 51200 x 5120 Q8 100 -> 50.4 (43.1), 5120 x 25600 Q8 55.1 -> 28.2 (21.6),
 // 2048 x 2048 bf16 7.2 -> 5.0 (1.3), 128256 x 4096 bf16 173 -> 160 (163); 16 tokens: 39.9 -> 33.1, 25.8 -> 19.8, 112 -> 58.5,
@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (warp == kConsumers / 32) {
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];\n" ::"l"(&wmap) : "memory");
+            if (!p.w_settled) pdl_wait();
             for (int stage = stage0, s = 0, lap = 0; stage < stage1; stage++) {
                 if (lap > 0 && !mbar_wait(empty(s), (lap - 1) & 1)) {
                     atomicExch(err, 15);

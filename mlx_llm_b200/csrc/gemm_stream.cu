@@ -166,9 +166,10 @@ __global__ void __launch_bounds__(kThreads) gemm_stream_kernel(const GemmParams 
         }
     };
 
-    // The weights do not depend on the kernel before this one: their first loads go out at once.  Everything else
+    // The weights of a model do not depend on the kernel before this one: their first loads go out at once.  Everything else
     // (activations, residual, the shared partial-sum scratch) waits for the previous grid to complete — this kernel
     // is launched with programmatic stream serialisation, so its CTAs may start while that grid's last CTAs finish.
+    if (!p.w_settled) pdl_wait();
     if (n_chunks > 0) {
 #pragma unroll
         for (int j = 0; j < PF; j++)

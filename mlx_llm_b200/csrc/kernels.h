@@ -57,6 +57,9 @@ struct GemmParams {
     // Optional (quantized): sbt[g * N + n] = scale(n, g) | bias(n, g) << 16, the scales and biases
     // transposed and interleaved so that the 32 feature rows of a warp read one 128-byte line per K group.
     const uint32_t* sbt;
+    // No kernel in front of this one writes the weights, so they may be read before those have completed: a model's own, and codes
+    // (only quantization kernels, launched the ordinary way, write those).  A caller's dense matrix may be the output of the call before.
+    bool w_settled;
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ float* gemm_f32_dst(const GemmParams& p, int t, int f) {

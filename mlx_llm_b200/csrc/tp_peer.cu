@@ -350,6 +350,7 @@ int32_t b2_tp_peer_projection(b2_tp_group* g, const uint16_t* x_dev, int32_t m, 
     GemmParams p{};
     p.x = x_dev;
     p.w = w_dev;
+    p.w_settled = bits != 0;
     p.scales = scales_dev;
     p.biases = biases_dev;
     p.bits = bits;

@@ -195,3 +195,29 @@ def test_q8_weights_are_rounded_as_dequantize_does(env, m, kernel):
     zero = (got & 0x7fff == 0) & (want & 0x7fff == 0)
     assert ((got == want) | zero).all()
     assert ((plain.download() == want) | zero).all()
+
+
+@pytest.mark.parametrize("rows", [32, 128])
+def test_weights_that_the_call_before_wrote(env, rows):
+    """A dense matrix that the projections in front have just written (by the ring kernel, by CTA pairs) is read whole by the ring
+    kernel and, 8-byte aligned activations, by the streaming kernel."""
+    ctx, K, orc, _lib = env
+    n, k, inner = 128, 2048, 4096
+    rng = np.random.default_rng(rows)
+    normal = lambda *shape: H.f32_to_bf16_np(rng.standard_normal(shape).astype(np.float32))
+    a, x = ctx.buf(normal(k, inner)), ctx.buf(normal(9, k))
+    sources = [[ctx.buf(normal(rows, inner)) for _ in range(n // rows)] for _ in range(2)]
+    w = ctx.buf(np.zeros((n, k), np.uint16))
+    outs = [ctx.empty((8, n), np.float32) for _ in range(2)]
+    want = []
+    for turn in range(12):
+        for at, source in enumerate(sources[turn & 1]):
+            K.linear(ctx, source, a, rows, k, inner, y_bf16=w.ptr + at * rows * k * 2)
+        x_at = x.ptr + (8 if turn & 2 else 0)
+        K.linear(ctx, x_at, w, 8, n, k, y_f32=outs[0])
+        ctx.sync()
+        K.linear(ctx, x_at, w, 8, n, k, y_f32=outs[1])  # (nothing in flight any more)
+        ctx.sync()
+        want.append(outs[1].download())
+        assert np.array_equal(outs[0].download(), want[-1])
+    assert not np.array_equal(want[0], want[1]) and np.array_equal(want[0], want[4])
