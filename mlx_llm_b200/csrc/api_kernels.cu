@@ -155,16 +155,22 @@ int32_t b2_projection(b2_ctx* ctx, const uint16_t* x_dev, const void* w_dev, con
     B2_REQUIRE((y_bf16_dev != nullptr) + (y_f32_dev != nullptr) + (h_dev != nullptr) == 1, B2_ERR_MSG, "b2_projection: one output buffer is wanted");
     GemmParams p{};
     if (bits) {
-        const size_t words = (size_t)out_dim * (in_dim / 64);
+        const int groups = in_dim / 64;
+        const size_t words = (size_t)out_dim * groups;
         void* scratch = nullptr;
-        int wide = 0;
-        B2_CHECK(b2_ctx_scratch(ctx, (words + 1) * 4, &scratch));
-        uint32_t* table = (uint32_t*)scratch;
-        B2_CUDA(cudaMemsetAsync(table + words, 0, 4, ctx->stream));
-        B2_CHECK(b2_gemm_build_sbt(ctx, scales_dev, biases_dev, out_dim, in_dim / 64, table, (int*)(table + words)));
-        B2_CUDA(cudaMemcpyAsync(&wide, table + words, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        uint32_t range[kTableRange];
+        B2_CHECK(b2_ctx_scratch(ctx, (words + kTableRange) * 4, &scratch));
+        uint32_t *table = (uint32_t*)scratch, *range_dev = table + words;
+        B2_CUDA(cudaMemsetAsync(range_dev, 0, sizeof(range), ctx->stream));
+        B2_CHECK(b2_gemm_table_range(ctx, scales_dev, biases_dev, out_dim, groups, range_dev));
+        B2_CUDA(cudaMemcpyAsync(range, range_dev, sizeof(range), cudaMemcpyDeviceToHost, ctx->stream));
         B2_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (!wide) p.sbt = table;
+        const int shift = b2_gemm_table_shift(range);
+        if (shift >= 0) {
+            B2_CHECK(b2_gemm_build_sbt(ctx, scales_dev, biases_dev, out_dim, groups, shift, table));
+            p.sbt = table;
+            p.sbt_unscale = std::ldexp(1.f, shift);
+        }
     }
     p.x = x_dev;
     p.w = w_dev;

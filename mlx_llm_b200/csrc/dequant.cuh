@@ -1,17 +1,16 @@
 // Group-quantized codes to bf16 weights without a conversion.
 //
 // An unsigned byte c in the low bits of a bf16, with nothing above it, IS the number c 2^-133 (up to 127 a subnormal, from 128 on the
-// exponent's lowest bit takes over where they end).  One fma with scale 2^93 and bias 2^-40 then gives bf16(c scale + bias) 2^-40;
+// exponent's lowest bit takes over where they end).  With scale 2^(133 - shift) and bias 2^-shift one fma gives the weight times 2^-shift;
 // the f32 sums are scaled back at the end.  A nibble in bits 4-7 counts 2^4 times as much.  Q4 weights are rounded once in every
 // projection kernel; Q8 weights are an f32 fma, then rounded to bf16 (b2_dequantize, the kernels without a table), and so they are here.
-// Exact for scales below 2^33 and weights above 2^-86; a matrix with a larger scale gets no table (b2_gemm_build_sbt) and stays with
-// the kernels that mask into 128 + c and subtract.
+//
+// The table of scales and biases holds them scaled.  A matrix's shift is the least with which its scales stay finite: 0 while all are
+// below 2^-5, which those of ordinary weights are, and then nothing is lost anywhere.  Up to 2^11 it is at most 16; every weight is
+// still exact (b2_gemm_table_shift refuses what is not), and f32 sums keep all their bits down to 2^-110.  A matrix that is refused
+// stays with the kernels that mask into 128 + c and subtract.
 #pragma once
 #include "common.cuh"
-
-constexpr uint32_t kByteUnit = 0x2b806e00u;    // (2^93, 2^-40) for a table word (scale, bias)
-constexpr uint32_t kNibbleUnit = 0x2b806c00u;  // (2^89, 2^-40)
-constexpr float kUnscale = 1099511627776.f;    // 2^40
 
 __device__ __forceinline__ uint32_t fma_bf2(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
@@ -28,7 +27,7 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     asm("prmt.b32 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
     return d;
 }
-// 8 Q4 codes in natural order: scales (scale 2^93, scale 2^89), three instructions a pair
+// 8 Q4 codes in natural order: scales (scale, scale 2^-4), three instructions a pair
 __device__ __forceinline__ void scaled_q4(uint32_t w, uint32_t scales, uint32_t b2, uint32_t (&out)[4]) {
     out[0] = fma_bf2(prmt(w, 0u, 0x4040u) & 0x00f0000fu, scales, b2);
     out[1] = fma_bf2(prmt(w, 0u, 0x4141u) & 0x00f0000fu, scales, b2);
@@ -62,5 +61,6 @@ __device__ __forceinline__ void scaled_q8_once(uint32_t w, uint32_t s2, uint32_t
 }
 // One fma in bf16 gives the bits of the two roundings unless the first drops a bias so small that code scale alone is a tie of the
 // second: never where the scale's exponent is at most 15 above the bias's (all mantissas, codes and signs tried; from 16 on 1 weight
-// in 70 000 differs, and more).  For a table word, the difference of its exponents times 2^23, less at most 2^15.
-__device__ __forceinline__ bool one_rounding(uint32_t sb) { return (int)((sb & 0x7f807f80u) * 0xffffu) < (16 << 23) - (1 << 15); }
+// in 70 000 differs, and more).  Taken where the fields differ by at most 8, since a subnormal bias lies up to 6 below its field.  For
+// a table word: the difference of its exponents, 133 apart already, times 2^23, less at most 2^15.
+__device__ __forceinline__ bool one_rounding(uint32_t sb) { return (int)((sb & 0x7f807f80u) * 0xffffu) < ((133 + 9) << 23) - (1 << 15); }

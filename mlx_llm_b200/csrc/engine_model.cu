@@ -172,31 +172,38 @@ int32_t set_local_dims(b2_model* m, b2_tp_group* tp) {
 // The projection kernels take scale and bias of a tile's feature rows at one K group as consecutive words: a second
 // copy of both, transposed and interleaved, makes that one line for 32 rows instead of 64.  (Not counted in weight_bytes: it is a
 // derived layout, 1/9 of the packed 4-bit codes.)
-static int32_t build_sbt(b2_model* m, Proj& p, int* wide_dev) {
-    if (p.bits == 0 || p.sbt) return B2_OK;
-    const int G = p.K / 64;
-    B2_CUDA(cudaMalloc((void**)&p.sbt, (size_t)p.N * G * 4));
-    m->allocs.push_back(p.sbt);
-    return b2_gemm_build_sbt(m->ctx, p.scales, p.biases, p.N, G, p.sbt, wide_dev);
+int32_t build_tables(b2_model* m) {
+    std::vector<Proj*> quantized;
+    for (auto& L : m->layers)
+        for (Proj* p : {&L.qkv, &L.o, &L.gu, &L.down})
+            if (p->bits != 0 && !p->sbt) quantized.push_back(p);
+    if (quantized.empty()) return B2_OK;
+    typedef uint32_t Range[kTableRange];
+    std::vector<uint32_t> ranges(quantized.size() * kTableRange);
+    void* ranges_dev = nullptr;
+    B2_CHECK(b2_ctx_scratch(m->ctx, ranges.size() * 4, &ranges_dev));
+    B2_CUDA(cudaMemsetAsync(ranges_dev, 0, ranges.size() * 4, m->ctx->stream));
+    for (size_t i = 0; i < quantized.size(); i++) {
+        const Proj& p = *quantized[i];
+        B2_CHECK(b2_gemm_table_range(m->ctx, p.scales, p.biases, p.N, p.K / 64, (uint32_t*)ranges_dev + i * kTableRange));
+    }
+    B2_CUDA(cudaMemcpyAsync(ranges.data(), ranges_dev, ranges.size() * 4, cudaMemcpyDeviceToHost, m->ctx->stream));
+    B2_CUDA(cudaStreamSynchronize(m->ctx->stream));
+    for (size_t i = 0; i < quantized.size(); i++) {
+        Proj& p = *quantized[i];
+        const int shift = b2_gemm_table_shift(*reinterpret_cast<const Range*>(ranges.data() + i * kTableRange));
+        if (shift < 0) continue;
+        B2_CUDA(cudaMalloc((void**)&p.sbt, (size_t)p.N * (p.K / 64) * 4));
+        m->allocs.push_back(p.sbt);
+        p.sbt_unscale = std::ldexp(1.f, shift);
+        B2_CHECK(b2_gemm_build_sbt(m->ctx, p.scales, p.biases, p.N, p.K / 64, shift, p.sbt));
+    }
+    return B2_OK;
 }
 
 int32_t finish_model(b2_model* m) {
-    const size_t tables = 4 * m->layers.size();
-    std::vector<int> wide(tables, 0);  // tables whose words cannot be scaled
-    void* flags = nullptr;
-    if (tables) {
-        B2_CHECK(b2_ctx_scratch(m->ctx, tables * sizeof(int), &flags));
-        B2_CUDA(cudaMemsetAsync(flags, 0, tables * sizeof(int), m->ctx->stream));
-    }
-    int* flag = (int*)flags;
-    for (auto& L : m->layers)
-        for (Proj* p : {&L.qkv, &L.o, &L.gu, &L.down}) B2_CHECK(build_sbt(m, *p, flag++));
-    if (tables) B2_CUDA(cudaMemcpyAsync(wide.data(), flags, tables * sizeof(int), cudaMemcpyDeviceToHost, m->ctx->stream));
+    B2_CHECK(build_tables(m));
     B2_CUDA(cudaStreamSynchronize(m->ctx->stream));
-    const int* found = wide.data();
-    for (auto& L : m->layers)
-        for (Proj* p : {&L.qkv, &L.o, &L.gu, &L.down})
-            if (*found++) p->sbt = nullptr;  // (its memory stays with the model's)
     m->inv_freq.resize(m->cfg.head_dim / 2);
     B2_CHECK(b2_rope_inv_freq(m->cfg.head_dim, m->cfg.rope_theta, m->cfg.rope_kind, m->cfg.rope_factor, m->cfg.rope_low_freq_factor,
                               m->cfg.rope_high_freq_factor, m->cfg.rope_original_context, m->inv_freq.data()));

@@ -121,6 +121,7 @@ int32_t gemm(b2_model* m, const Proj& p, const uint16_t* x, int M, int ldx, uint
     g.scales = p.scales;
     g.biases = p.biases;
     g.sbt = p.sbt;
+    g.sbt_unscale = p.sbt_unscale;
     g.w_settled = true;
     g.bits = p.bits;
     g.group = 64;
@@ -147,6 +148,7 @@ int32_t gemm_reduce_residual(b2_model* m, const Proj& p, const uint16_t* a, int 
     g.scales = p.scales;
     g.biases = p.biases;
     g.sbt = p.sbt;
+    g.sbt_unscale = p.sbt_unscale;
     g.w_settled = true;
     g.bits = p.bits;
     g.group = 64;

@@ -178,12 +178,8 @@ __global__ void __launch_bounds__(kThreads, 2)
                 if (WK)
 #pragma unroll
                     for (int i = 0; i < 2; i++) {
-                        const uint32_t lo = mul_bf2(sb[sp][i], kByteUnit);
-                        s_lo[i] = prmt(lo, lo, 0x1010u), b2[i] = prmt(lo, lo, 0x3232u);
-                        if (WK == 4) {
-                            const uint32_t hi = mul_bf2(sb[sp][i], kNibbleUnit);
-                            s_hi[i] = prmt(hi, hi, 0x1010u);
-                        }
+                        s_lo[i] = prmt(sb[sp][i], 0u, 0x1010u), b2[i] = prmt(sb[sp][i], 0u, 0x3232u);
+                        if (WK == 4) s_hi[i] = mul_bf2(s_lo[i], 0x3d803d80u);  // 2^-4
                     }
 #pragma unroll
                 for (int e8 = 0; e8 < R::E / 8; e8++) {  // eight K of every row: two MMA steps
@@ -248,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(at + (uint32_t)((nt * 8 + 2 * t + (e & 1)) * kSumStride + (e >> 1) * 8 + row) * 4u),
-                                 "f"(WK ? acc[nt][e] * kUnscale : acc[nt][e])
+                                 "f"(WK ? acc[nt][e] * p.sbt_unscale : acc[nt][e])
                                  : "memory");
                     acc[nt][e] = 0.f;
                 }

@@ -43,6 +43,8 @@
 // falls through to the common exit, where the TMEM columns are freed.
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "dequant.cuh"
 #include "kernels.h"
@@ -258,7 +260,7 @@ __device__ __forceinline__ Piece piece_at(int unit, int unit_end, int bpt, int b
 
 // With the table a weight costs 1.5 instructions (Q4) or 2 (Q8) instead of 2.4 and 3.5 (dequant.cuh): steps of the 8B Q4 model with 64
 // sequences 6.52 -> 6.27 ms, with 96 and a 512-token portion 13.56 -> 13.25, the 32B Q8 model's 512-token portion (8 layers) 8.25 -> 7.94.
-template <int WK, int EPI, bool TABLE>  // TABLE: scales and biases come as GemmParams::sbt, whose words may be scaled (dequant.cuh)
+template <int WK, int EPI, bool TABLE>  // TABLE: scales and biases come as GemmParams::sbt, whose words are scaled (dequant.cuh)
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_tc_pair_kernel(const GemmParams p, const PairPlan plan, const __grid_constant__ CUtensorMap map_x,
                         const __grid_constant__ CUtensorMap map_x_small, const __grid_constant__ CUtensorMap map_w) {
@@ -391,9 +393,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         break;
                     }
                     if (TABLE) {
-                        const uint32_t b2 = mul_bf2(cbi * 0x10001u, 0x2b802b80u);
                         if (WK == 4) {
-                            const uint32_t scales = mul_bf2(csc * 0x10001u, 0x6c006e00u);
+                            const uint32_t scales = mul_bf2(csc * 0x10001u, 0x3d803f80u), b2 = cbi * 0x10001u;  // (1, 2^-4)
 #pragma unroll
                             for (int i = 0; i < 8; i++) {
                                 uint32_t o[4];
@@ -401,7 +402,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                                 sts128(sA + ((((uint32_t)i) ^ sw) << 4), o[0], o[1], o[2], o[3]);
                             }
                         } else {
-                            const float sf = bflo(mul_bf2(csc, 0x6e00u)), bf = bflo(b2);
+                            const float sf = bflo(csc), bf = bflo(cbi);
 #pragma unroll
                             for (int i = 0; i < 8; i++) {
                                 uint32_t o[4];
@@ -509,7 +510,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     for (int i = 0; i < 32; i++) {
                         if (i >= left) break;
                         const int t = tg + i;
-                        const float a = TABLE ? __uint_as_float(v[i]) * kUnscale : __uint_as_float(v[i]);
+                        const float a = TABLE ? __uint_as_float(v[i]) * p.sbt_unscale : __uint_as_float(v[i]);
                         if (splits > 1) {
                             plan.partial[((size_t)pc.split * M + t) * N + f] = a;
                         } else if (EPI == EPI_F32) {
@@ -777,17 +778,28 @@ int32_t get_map(b2_ctx* ctx, const void* ptr, uint64_t rows, uint64_t k, uint64_
     return B2_OK;
 }
 
-__global__ void sbt_build_kernel(const uint16_t* __restrict__ scales, const uint16_t* __restrict__ biases, int N, int G, uint32_t* __restrict__ sbt,
-                                 int* __restrict__ wide) {
+// largest scale, largest bias, and 0x7fff less the smallest number of both that is not zero, as bits without the sign
+__global__ void table_range_kernel(const uint16_t* __restrict__ scales, const uint16_t* __restrict__ biases, int64_t count, uint32_t* __restrict__ range) {
+    uint32_t scale = 0, bias = 0, small = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t s = scales[i] & 0x7fffu, b = biases[i] & 0x7fffu;
+        scale = max(scale, s), bias = max(bias, b);
+        if (s) small = max(small, 0x7fffu - s);
+        if (b) small = max(small, 0x7fffu - b);
+    }
+    scale = __reduce_max_sync(0xffffffffu, scale), bias = __reduce_max_sync(0xffffffffu, bias), small = __reduce_max_sync(0xffffffffu, small);
+    if ((threadIdx.x & 31) == 0) atomicMax(range, scale), atomicMax(range + 1, bias), atomicMax(range + 2, small);
+}
+
+__global__ void sbt_build_kernel(const uint16_t* __restrict__ scales, const uint16_t* __restrict__ biases, int N, int G, int shift, uint32_t* __restrict__ sbt) {
     // 32 x 32 tiles through shared memory: coalesced reads along the groups of a row, coalesced writes along the rows
     __shared__ uint32_t tile[32][33];
     const int g0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         const int n = n0 + r, g = g0 + threadIdx.x;
         if (n < N && g < G) {
-            const uint32_t scale = scales[(size_t)n * G + g];
-            if ((scale & 0x7f80u) >= 0x5000u) *wide = 1;  // 2^33 and more
-            tile[r][threadIdx.x] = scale | ((uint32_t)biases[(size_t)n * G + g] << 16);
+            const size_t i = (size_t)n * G + g;
+            tile[r][threadIdx.x] = (uint32_t)f2bf(ldexpf(bf2f(scales[i]), 133 - shift)) | ((uint32_t)f2bf(ldexpf(bf2f(biases[i]), -shift)) << 16);
         }
     }
     __syncthreads();
@@ -895,8 +907,25 @@ int32_t dispatch_pair(b2_ctx* ctx, const GemmParams& p, int* err) {
 
 }  // namespace
 
-int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev, int* wide_dev) {
-    sbt_build_kernel<<<dim3((unsigned)((G + 31) / 32), (unsigned)((N + 31) / 32)), dim3(32, 8), 0, ctx->stream>>>(scales_dev, biases_dev, N, G, sbt_dev, wide_dev);
+int32_t b2_gemm_table_range(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* range_dev) {
+    const int64_t count = (int64_t)N * G;
+    table_range_kernel<<<(unsigned)std::min<int64_t>((count + 1023) / 1024, 4 * ctx->sm_count), 256, 0, ctx->stream>>>(scales_dev, biases_dev, count, range_dev);
+    B2_LAUNCHED(ctx);
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
+
+int b2_gemm_table_shift(const uint32_t (&range)[kTableRange]) {
+    const int scale = (int)(range[0] >> 7), bias = (int)(range[1] >> 7), small = (int)((0x7fffu - range[2]) >> 7);  // exponent fields
+    const int shift = std::max(0, scale - 127 + 6);  // scale 2^(133 - shift) below 2^128
+    if (shift == 0) return 0;
+    // The last bit of the smallest number, 7 below its exponent, has to stay at 2^-133 or above it: then all weights, multiples of it, are
+    // exact wherever they are smaller than what bf16 holds in full.  And no weight may have been infinite for its size.
+    return shift <= 16 && small > shift && bias < 254 ? shift : -1;
+}
+
+int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, int shift, uint32_t* sbt_dev) {
+    sbt_build_kernel<<<dim3((unsigned)((G + 31) / 32), (unsigned)((N + 31) / 32)), dim3(32, 8), 0, ctx->stream>>>(scales_dev, biases_dev, N, G, shift, sbt_dev);
     B2_LAUNCHED(ctx);
     B2_CUDA(cudaGetLastError());
     return B2_OK;

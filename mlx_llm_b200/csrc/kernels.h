@@ -54,9 +54,11 @@ struct GemmParams {
     // sum to the rank that will add it up.  f32_chunk is a multiple of 4.
     float* out_f32_by_chunk[8];
     int f32_chunk;
-    // Optional (quantized): sbt[g * N + n] = scale(n, g) | bias(n, g) << 16, the scales and biases
-    // transposed and interleaved so that the 32 feature rows of a warp read one 128-byte line per K group.
+    // Optional (quantized): sbt[g * N + n] = scale(n, g) 2^(133 - shift) | bias(n, g) 2^-shift << 16, the scales and biases as the
+    // kernels that convert codes as numbers want them (dequant.cuh), transposed and interleaved so that the 32 feature rows of a warp
+    // read one 128-byte line per K group; sbt_unscale = 2^shift.
     const uint32_t* sbt;
+    float sbt_unscale;
     // No kernel in front of this one writes the weights, so they may be read before those have completed: a model's own, and codes
     // (only quantization kernels, launched the ordinary way, write those).  A caller's dense matrix may be the output of the call before.
     bool w_settled;
@@ -93,10 +95,13 @@ int32_t b2_gemm_ring_launch(b2_ctx* ctx, const GemmParams& p, int* cluster = nul
 // tcgen05 / TMEM path, CTA-pair form (gemm_tc.cu): taken by b2_gemm_launch when eligible.
 bool b2_gemm_tc_eligible(const GemmParams& p);
 int32_t b2_gemm_tc_launch(b2_ctx* ctx, const GemmParams& p);
-// Fills sbt (N * G words) from scales / biases [N, G] (see GemmParams::sbt); enqueued on the context's stream.  *wide_dev becomes 1
-// when a scale is 2^33 or more in size, infinite or not a number: such a table must not be used, since the kernels that take it
-// scale its words by powers of two (dequant.cuh).
-int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* sbt_dev, int* wide_dev);
+// The table of a quantized matrix (GemmParams::sbt), N * G words, in three steps, all on the context's stream: what sizes its scales and
+// biases have (range_dev: kTableRange words, zero before); on the host the shift that follows, -1 where the matrix can have no table;
+// the table.
+constexpr int kTableRange = 3;
+int32_t b2_gemm_table_range(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, uint32_t* range_dev);
+int b2_gemm_table_shift(const uint32_t (&range)[kTableRange]);
+int32_t b2_gemm_build_sbt(b2_ctx* ctx, const uint16_t* scales_dev, const uint16_t* biases_dev, int N, int G, int shift, uint32_t* sbt_dev);
 
 // ---- elementwise / normalisation / embedding / sampling (fused_ops.cu) ---------------------------
 // out = rmsnorm(x) * w, one row per token; rows gathered through `row_idx` when non-null.

@@ -221,3 +221,41 @@ def test_weights_that_the_call_before_wrote(env, rows):
         want.append(outs[1].download())
         assert np.array_equal(outs[0].download(), want[-1])
     assert not np.array_equal(want[0], want[1]) and np.array_equal(want[0], want[4])
+
+
+# exponents of scales and biases: lowest and highest; whether a table is possible; the size of the activations
+TABLE_RANGES = {"ordinary": (-14, -8, True, 0), "smallest": (-133, -120, True, 0), "small_sums": (-30, -20, True, -90), "largest_unshifted": (-126, -6, True, 0),
+                "shifted": (-125, -5, True, 0), "shifted_most": (-110, 10, True, 0), "too_large": (-8, 11, False, 0), "too_wide": (-111, 10, False, 0)}
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("m", [7, 64])
+@pytest.mark.parametrize("name", TABLE_RANGES)
+def test_table_of_any_size_of_scales(env, name, m, bits):
+    """The kernels that read the scaled table give the bits of those that read scales and biases themselves, from subnormal scales to
+    the largest that get a table, sums near the lower end of f32 too; matrices beyond take the other kernels."""
+    ctx, K, orc, _lib = env
+    lo, hi, possible, size = TABLE_RANGES[name]
+    n, k = 256, 512
+    rng = np.random.default_rng(m)
+
+    def numbers():
+        e = rng.integers(max(lo, -126), hi + 1, (n, k // 64))
+        e[0, 0], e[1, 1] = hi, max(lo, -126)
+        v = np.ldexp(1 + rng.integers(0, 128, e.shape) / 128, e) * rng.choice([-1.0, 1.0], e.shape)
+        if lo < -126:
+            v[2::3] = np.ldexp(rng.integers(1, 128, v[2::3].shape), -133)  # subnormal
+        return H.f32_to_bf16_np(v.astype(np.float32))
+
+    packed = rng.integers(0, 2**32, size=(n, k * bits // 32), dtype=np.uint32)
+    scales, biases = numbers(), numbers()
+    x = H.f32_to_bf16_np(np.ldexp(rng.standard_normal((m, k)), size).astype(np.float32))
+    dx, dp, ds, db = ctx.buf(x), ctx.buf(packed), ctx.buf(scales), ctx.buf(biases)
+    with_table, without = ctx.empty((m, n), np.float32), ctx.empty((m, n), np.float32)
+    route = K.projection(ctx, dx, dp, ds, db, m, n, k, bits, y_f32=with_table)
+    assert route[:2] == (3 if m > 32 else 2 if possible else 1, int(possible))
+    K.qmm(ctx, dx, dp, ds, db, m, n, k, bits, None, without)
+    ctx.sync()
+    want = without.download()
+    assert np.isfinite(want).all() and np.abs(want).max() > 0
+    assert np.array_equal(with_table.download(), want)
