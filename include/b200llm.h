@@ -413,7 +413,9 @@ int32_t b2_cache_gather_f32(b2_cache* c, int32_t layer, float* k_host, float* v_
 /* One forward over a ragged batch: sequence i contributes n_tokens[i] ids at positions
  * offset(caches[i])..; returns last-position logits [num_seqs, vocab] (bf16; f32 for an f32 model) on the host and advances
  * the caches.  Covers Decode::step (src/decode/stream.rs:22-29), CausalLm::decode_logits
- * (llama.rs:351-370) and decode_logits_per_seq (llama.rs:530-558).  When the call fails, what logits_host holds is undefined. */
+ * (llama.rs:351-370) and decode_logits_per_seq (llama.rs:530-558).  A step that is abandoned (B2_ERR_TIMEOUT) leaves logits_host and
+ * argmax_host as they are.  Logits go straight into page-locked memory (b2_host_alloc_pinned); pageable memory costs the call a copy
+ * by the host (0.6 ms for 64 rows of 128256 bf16 logits). */
 int32_t b2_model_step(b2_model* m, const int32_t* ids_host, const int32_t* n_tokens, int32_t num_seqs, b2_cache** caches,
                       void* logits_host /* nullable; uint16_t (bf16) rows, float rows for an f32 model */,
                       int32_t* argmax_host /* nullable */);

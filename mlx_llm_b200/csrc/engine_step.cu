@@ -490,25 +490,28 @@ int32_t b2_engine_forward(b2_model* m, std::vector<SeqStep>& seqs, void* logits_
         B2_CHECK(forward_bf16_layers(m, pool, mo, in, ids_dev, T, n_dec, dec_ctx_sum, W, P, pf_flops, pf_max_ctx, chunk_tiles, q_tile, n_logits, logit_rows));
     }
     const int lsz = m->logits_f32() ? 4 : 2;
-    // Logits go straight into a page-locked buffer of the caller; a pageable one gets them through a page-locked buffer of the model.
-    // The host's copy between the two was 0.6 ms of a 64-sequence step (128256 bf16 logits each), 0.9 ms of a 97-sequence one.
+    // Logits go straight into a page-locked buffer of the caller, once the step is known to be whole; a pageable one gets them through a
+    // page-locked buffer of the model.  The host's copy between the two was 0.6 ms of a 64-sequence step (128256 bf16 logits each),
+    // 0.9 ms of a 97-sequence one.
     const size_t logits_bytes = (size_t)n_logits * c.vocab_size * lsz;
     const bool direct = logits_out && logits_bytes && pinned_range(logits_out, logits_bytes);
+    auto copy_logits = [&](void* to) {
+        m->d2h_bytes += (int64_t)logits_bytes;
+        return cudaMemcpy2DAsync(to, (size_t)c.vocab_size * lsz, m->logits_f32() ? (const void*)logits_f32_dev : (const void*)w.logits,
+                                 (size_t)logits_ld * lsz, (size_t)c.vocab_size * lsz, (size_t)n_logits, cudaMemcpyDeviceToHost, st);
+    };
     if (n_logits > 0) {
         b2_prof_mark(ctx, B2_CLS_META);
         B2_CUDA(cudaMemcpyAsync(w.argmax_host, w.argmax, (size_t)n_logits * 4, cudaMemcpyDeviceToHost, st));
         m->d2h_bytes += (int64_t)n_logits * 4;
-        if (logits_out) {
-            const size_t bytes = logits_bytes;
-            if (!direct && bytes > w.logits_host_cap) {
+        if (logits_out && !direct) {
+            if (logits_bytes > w.logits_host_cap) {
                 B2_CUDA(cudaStreamSynchronize(st));
                 if (w.logits_host) cudaFreeHost(w.logits_host);
-                B2_CUDA(cudaHostAlloc((void**)&w.logits_host, bytes, cudaHostAllocDefault));
-                w.logits_host_cap = bytes;
+                B2_CUDA(cudaHostAlloc((void**)&w.logits_host, logits_bytes, cudaHostAllocDefault));
+                w.logits_host_cap = logits_bytes;
             }
-            B2_CUDA(cudaMemcpy2DAsync(direct ? logits_out : w.logits_host, (size_t)c.vocab_size * lsz, m->logits_f32() ? (const void*)logits_f32_dev : (const void*)w.logits,
-                                      (size_t)logits_ld * lsz, (size_t)c.vocab_size * lsz, (size_t)n_logits, cudaMemcpyDeviceToHost, st));
-            m->d2h_bytes += (int64_t)bytes;
+            B2_CUDA(copy_logits(w.logits_host));
         }
     }
     // the error word a bounded device-side wait raises travels back with the sampled ids
@@ -517,6 +520,15 @@ int32_t b2_engine_forward(b2_model* m, std::vector<SeqStep>& seqs, void* logits_
     b2_prof_mark(ctx, -1);
     B2_CUDA(cudaEventRecord(m->ev1, st));
     B2_CUDA(cudaStreamSynchronize(st));
+    if (direct && ctx->err_host[0] == 0) {
+        b2_prof_mark(ctx, B2_CLS_META);
+        const cudaError_t copied = copy_logits(logits_out);
+        b2_prof_mark(ctx, -1);
+        const cudaError_t marked = cudaEventRecord(m->ev1, st);
+        B2_CUDA(cudaStreamSynchronize(st));  // (before anything may return: the buffer is the caller's)
+        B2_CUDA(copied);
+        B2_CUDA(marked);
+    }
     B2_CUDA(cudaGetLastError());
     b2_prof_collect(ctx);
     float ms = 0.f;

@@ -577,3 +577,94 @@ def test_nvtx_ranges_do_not_change_a_step(env):
     ctx.nvtx(False)
     assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1]) and outs[0][2] == outs[1][2]
 
+
+
+def step_into(eng, model, caches, ids, address, tokens):
+    """b2_model_step with the logits at a host address."""
+    import ctypes as C
+
+    from mlx_llm_b200 import _lib
+
+    flat, n = np.concatenate(ids).astype(np.int32), np.array([len(i) for i in ids], np.int32)
+    handles = (C.c_void_p * len(ids))(*[c.h for c in caches])
+    _lib.check(_lib.load().b2_model_step(model.h, _lib.ptr(flat), _lib.ptr(n), len(ids), handles, C.c_void_p(address), _lib.ptr(tokens)))
+
+
+@pytest.mark.parametrize("memory", ["pageable", "page_locked", "page_locked_inside", "registered"])
+def test_logits_into_any_host_memory(env, memory):
+    """The same logits wherever the caller's buffer lies, and nothing beside them is written."""
+    import ctypes as C
+
+    from mlx_llm_b200 import _lib
+
+    ctx, eng, orc, model, omodel = env
+    lib, prompts = _lib.load(), H.config0_prompts()
+    pool = eng.BlockPool(ctx, model, 16, 64, 4, 16)
+    caches = [eng.PagedKvCache(pool) for _ in prompts]
+    want, tokens = model.step(list(zip(prompts, caches)))
+    room = 4096 + want.nbytes + 4096
+    inner = {"page_locked": 0, "page_locked_inside": 1030}.get(memory, 64)  # (rows of any alignment)
+    if memory.startswith("page_locked"):
+        address = C.c_void_p()
+        _lib.check(lib.b2_host_alloc_pinned(C.c_size_t(room), C.byref(address)))
+        base = address.value
+    else:
+        own = np.zeros(room + 4096, np.uint8)
+        base = (own.ctypes.data + 4095) // 4096 * 4096
+    raw = np.ctypeslib.as_array((C.c_uint8 * room).from_address(base))
+    cudart = C.CDLL("libcudart.so.12") if memory == "registered" else None
+    if cudart:
+        assert cudart.cudaHostRegister(C.c_void_p(base), C.c_size_t(room), 0) == 0
+    try:
+        raw[:] = 0xa5
+        for c in caches:
+            c.reset()
+        again = np.empty(len(prompts), np.int32)
+        step_into(eng, model, caches, prompts, base + inner, again)
+        assert raw[inner:inner + want.nbytes].tobytes() == want.tobytes() and np.array_equal(again, tokens)
+        assert (raw[:inner] == 0xa5).all() and (raw[inner + want.nbytes:] == 0xa5).all()
+    finally:
+        if cudart:
+            assert cudart.cudaHostUnregister(C.c_void_p(base)) == 0
+        if memory.startswith("page_locked"):
+            _lib.check(lib.b2_host_free_pinned(C.c_void_p(base)))
+
+
+@pytest.mark.parametrize("page_locked", [False, True])
+def test_abandoned_step_leaves_the_callers_buffers(page_locked):
+    """A wait that ran out (a reduction whose other rank never comes, with a short limit) is pending when the step ends: the step is
+    abandoned, no cache advances, and neither logits nor tokens are written; the next step is whole again."""
+    import ctypes as C
+
+    from mlx_llm_b200 import _lib, engine as eng
+
+    ctx, lib = _lib.Context(0), _lib.load()
+    model = H.build_engine_model(eng, ctx)
+    prompts = H.config0_prompts()
+    pool = eng.BlockPool(ctx, model, 16, 64, 4, 16)
+    caches = [eng.PagedKvCache(pool) for _ in prompts]
+    groups = [eng.TpGroup(ctx, None, r, 2) for r in range(2)]
+    for g in groups:
+        g.peer_alloc(64, 256)
+    eng.TpGroup.peer_attach_local(groups)
+    rows = len(prompts)
+    nbytes = rows * model.config().vocab_size * 2
+    address = C.c_void_p()
+    _lib.check(lib.b2_host_alloc_pinned(C.c_size_t(nbytes), C.byref(address)))
+    raw = np.ctypeslib.as_array((C.c_uint8 * nbytes).from_address(address.value)) if page_locked else np.empty(nbytes, np.uint8)
+    tokens = np.full(rows, -7, np.int32)
+    raw[:] = 0xa5
+    _lib.check(lib.b2_ctx_set_wait_limit_ms(ctx.h, 50))
+    groups[0].peer_reduce_residual(64)
+    with pytest.raises(_lib.B2Error) as e:
+        step_into(eng, model, caches, prompts, raw.ctypes.data, tokens)
+    assert e.value.code == -9  # B2_ERR_TIMEOUT
+    assert (raw == 0xa5).all() and (tokens == -7).all() and [c.offset() for c in caches] == [0] * rows
+    step_into(eng, model, caches, prompts, raw.ctypes.data, tokens)
+    assert (raw != 0xa5).any() and (tokens >= 0).all() and [c.offset() for c in caches] == [len(p) for p in prompts]
+    del raw
+    for g in groups:
+        g.free()
+    _lib.check(lib.b2_host_free_pinned(address))
+    model.free()
+    ctx.close()
