@@ -14,8 +14,8 @@
 //                the group on N:  S^T = K Q^T, then O^T += V^T P^T.  P^T reaches the B-operand
 //                layout with one movmatrix per 8 tokens.  Softmax statistics are per column,
 //                reduced with three xor-shuffles.
-//   merge      = per-CTA cross-warp log-sum-exp merge in shared memory; chunks of a sequence are
-//                merged by a second small kernel (skipped for single-chunk sequences).
+//   merge      = per-CTA cross-warp log-sum-exp merge in shared memory; the CTA that finishes last for a (sequence, kv head)
+//                merges its chunks in order (no CTA waits for another).
 // This is HBM-bound byte streaming: the tensor cores are used only to keep the CUDA cores off the
 // critical path, so no tcgen05/TMEM here.
 #include <cfloat>
@@ -334,9 +334,8 @@ __device__ __forceinline__ void decode_item(const DecodeAttnParams& p, uint8_t* 
 // (item, kv head) pair: the whole operation is one launch.
 constexpr int kInlineSeqs = 1024;
 
-// kStages: tiles that a warp has on their way.  Two let three blocks on an SM instead of two, which batches gain from (64 sequences 54.5 -> 52.2 us a
-// layer); where all blocks fit the machine at once anyway, three are as before (one sequence: 8.5 us, with two 9.2, and less room
-// for the projection behind it).
+// kStages: tiles that a warp has on their way.  Two let three blocks on an SM instead of two, which batches gain from (64 sequences 54.5
+// -> 52.2 us a layer); which where: two_tiles().
 template <int HD, int kStages>
 __global__ void __launch_bounds__(kWarps * 32) paged_attn_decode_kernel(const DecodeAttnParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -449,14 +448,28 @@ __global__ void decode_worklist_kernel(const int32_t* ctx_lens, int num_seqs, in
     }
 }
 
+// Head size 128: two tiles a warp (three blocks on an SM) or three (two blocks).  `blocks` with work at most, of a list that the host has
+// made or of the one in the kernel, whose grid is larger and, but for that work, ends at once.
+//   list of the host: three where all blocks fit the machine together (one sequence of the 8B model 8.5 us, with two tiles 9.2).
+//   list in the kernel: two get the idle blocks out of the way sooner (8 x 128 tokens 8.7 -> 6.6 us, 8 x 512 12.5 -> 10.3, 16 x 64-1500
+//   22.4 -> 17.5, 1 x 128 7.8 -> 6.9); three for few long sequences, of at least 32 chunks each (1 x 4096 13.1 -> 12.3, 4 x 9000 with one
+//   kv head 21.6 -> 20.3; 1 x 32000 in 512-token chunks, 472 items on 444 or 296 places, 47.8 -> 43.4).
+bool two_tiles(long blocks, const DecodeAttnParams& p, int sm_count) {
+    if (p.work_seq) return blocks > 2l * sm_count;
+    const long chunks = ((long)p.max_blocks * p.page_tiles + p.chunk_tiles - 1) / p.chunk_tiles;
+    return chunks < 32 || blocks > 4l * sm_count;
+}
+
 template <int HD, int kStages>
 int32_t launch_decode(b2_ctx* ctx, const DecodeAttnParams& p, int grid_work, int num_seqs) {
     const int smem = smem_bytes(HD, kStages);
     B2_SMEM_ONCE(ctx, (paged_attn_decode_kernel<HD, kStages>), smem);
     dim3 grid(grid_work, p.hkv);
-    // in-kernel work list: a fixed grid of sixteen CTAs per SM, each taking every gridDim.x-th item.  Two are resident
-    // per SM at a time and none waits for another, so the rest simply queue; the fine grain lets the hardware's block
-    // scheduler even out items of different cost (measured: 4 / 8 / 16 CTAs per SM -> 174 / 150 / 137 us on 64 sequences)
+    // in-kernel work list: a fixed grid of sixteen CTAs per SM, each taking every gridDim.x-th item.  Two or three are
+    // resident per SM at a time and none waits for another, so the rest simply queue; the fine grain lets the hardware's
+    // block scheduler even out items of different cost (measured with three tiles a warp: 4 / 8 / 16 CTAs per SM -> 174 / 150 / 137 us
+    // on 64 sequences).  Only as many CTAs as there can be items: a few short sequences gain up to 25 %, but the kernel behind then
+    // takes the free SMs sooner, and one sequence of 4096 with a projection behind it goes from 21.0 to 23.2 us.
     if (!p.work_seq) grid = dim3(16 * ctx->sm_count);
     B2_CUDA(b2_launch_pdl(ctx->pdl_consumers, paged_attn_decode_kernel<HD, kStages>, grid, dim3(kWarps * 32), (size_t)smem, ctx->stream, p));
     B2_LAUNCHED(ctx);
@@ -496,8 +509,7 @@ int32_t b2_decode_attn_launch(b2_ctx* ctx, const DecodeAttnParams& p, int head_d
     B2_REQUIRE(p.merge_counters, B2_ERR_MSG, "paged_attn_decode: no arrival counters for the merge");
     B2_REQUIRE(p.work_seq || (p.num_seqs >= 1 && p.num_seqs <= kInlineSeqs), B2_ERR_MSG, "paged_attn_decode: no work list and too many sequences to derive one in the kernel");
     if (grid_work <= 0 || num_seqs <= 0) return B2_OK;
-    const bool many = !p.work_seq || (long)grid_work * p.hkv > 2l * ctx->sm_count;
-    if (head_dim == 128) return many ? launch_decode<128, 2>(ctx, p, grid_work, num_seqs) : launch_decode<128, 3>(ctx, p, grid_work, num_seqs);
+    if (head_dim == 128) return two_tiles((long)grid_work * p.hkv, p, ctx->sm_count) ? launch_decode<128, 2>(ctx, p, grid_work, num_seqs) : launch_decode<128, 3>(ctx, p, grid_work, num_seqs);
     if (head_dim == 64) return launch_decode<64, 3>(ctx, p, grid_work, num_seqs);
     return b2_fail(B2_ERR_UNSUPPORTED, "paged_attn_decode: head_dim must be 64 or 128");
 }
@@ -607,8 +619,7 @@ namespace {
 // threads that make their FIRST call on one device at the same moment both run the set-up and store the
 // same values, which is harmless; after that the call only reads them.
 unsigned char* g_scratch_addr[64] = {};
-bool g_static_smem_set[64][2] = {};
-int g_static_grid[64][2] = {};  // sixteen CTAs per SM of the device
+int g_static_sms[64] = {};
 }  // namespace
 
 extern "C" int32_t b2_paged_attn_decode_static(void* stream, const uint16_t* q_dev, const uint16_t* k_pool_dev,
@@ -645,21 +656,16 @@ extern "C" int32_t b2_paged_attn_decode_static(void* stream, const uint16_t* q_d
         B2_CUDA(cudaGetSymbolAddress((void**)&ptr, g_decode_scratch));
         g_scratch_addr[dev] = ptr;
     }
-    const int smem = head_dim == 128 ? smem_bytes(128, 2) : smem_bytes(64, 3);
-    if (!g_static_smem_set[dev][head_dim == 128]) {
-        if (head_dim == 128)
-            B2_CUDA(cudaFuncSetAttribute(paged_attn_decode_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        else
-            B2_CUDA(cudaFuncSetAttribute(paged_attn_decode_kernel<64, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        g_static_smem_set[dev][head_dim == 128] = true;
+    if (!g_static_sms[dev]) {
+        B2_CUDA(cudaFuncSetAttribute(paged_attn_decode_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(128, 2)));
+        B2_CUDA(cudaFuncSetAttribute(paged_attn_decode_kernel<128, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(128, 3)));
+        B2_CUDA(cudaFuncSetAttribute(paged_attn_decode_kernel<64, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(64, 3)));
+        int sms = 0;
+        B2_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        g_static_sms[dev] = sms;
     }
     unsigned char* scratch = g_scratch_addr[dev];
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (!g_static_grid[dev][head_dim == 128]) {
-        int sms = 0;
-        B2_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        g_static_grid[dev][head_dim == 128] = 16 * sms;
-    }
     DecodeAttnParams p{};
     p.q = q_dev;
     p.k_pool = k_pool_dev;
@@ -680,11 +686,13 @@ extern "C" int32_t b2_paged_attn_decode_static(void* stream, const uint16_t* q_d
     p.part_o = reinterpret_cast<float*>(scratch + kStaticCounterBytes);
     p.part_ml = p.part_o + (size_t)max_work * hq * head_dim;
     p.out = out_dev;
-    const dim3 grid((unsigned)g_static_grid[dev][head_dim == 128]);
-    if (head_dim == 128)
-        paged_attn_decode_kernel<128, 2><<<grid, kWarps * 32, smem, st>>>(p);
+    const dim3 grid((unsigned)(16 * g_static_sms[dev]));
+    if (head_dim == 64)
+        paged_attn_decode_kernel<64, 3><<<grid, kWarps * 32, smem_bytes(64, 3), st>>>(p);
+    else if (two_tiles(max_work * hkv, p, g_static_sms[dev]))
+        paged_attn_decode_kernel<128, 2><<<grid, kWarps * 32, smem_bytes(128, 2), st>>>(p);
     else
-        paged_attn_decode_kernel<64, 3><<<grid, kWarps * 32, smem, st>>>(p);
+        paged_attn_decode_kernel<128, 3><<<grid, kWarps * 32, smem_bytes(128, 3), st>>>(p);
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }

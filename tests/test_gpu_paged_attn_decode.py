@@ -129,3 +129,23 @@ def test_decode_linearity_full_size(env):
                               case["scale"])
     err = np.abs(outs[0] - ref).max(axis=(1, 2))
     assert err.shape == (64,) and err.max() <= TOL, f"worst sequence {int(err.argmax())}: max-abs {err.max()}"
+
+
+@pytest.mark.parametrize("lens", [[4100], [4096, 3000, 17]])
+def test_decode_variants_agree(env, lens):
+    """Few long sequences take another number of tiles a warp than the same sequences with wide block tables: the same bits."""
+    ctx, kernels, orc = env
+    case = H.make_paged_case(17, lens, 8, 2, 128, 16)
+    dev = {k: ctx.buf(case[k]) for k in ("q", "kpool", "vpool", "ctx_lens")}
+    outs = []
+    for blocks in (case["max_blocks"], 32 * case["max_blocks"]):
+        table = np.zeros((len(lens), blocks), np.int32)
+        table[:, :case["max_blocks"]] = case["block_tables"]
+        o = ctx.empty(case["q"].shape, np.uint16)
+        kernels.paged_attn_decode(ctx, dev["q"], dev["kpool"], dev["vpool"], ctx.buf(table), dev["ctx_lens"], len(lens), 8, 2, 128, 16, case["scale"], o,
+                                  blocks, 128)
+        ctx.sync()
+        outs.append(o.download())
+    assert np.array_equal(*outs)
+    ref = orc.paged_attention(case["q"], case["kpool"], case["vpool"], case["block_tables"], case["cu_seqlens"], case["ctx_lens"], case["scale"])
+    assert H.close_bf16_out(outs[0], ref, TOL)[0]
