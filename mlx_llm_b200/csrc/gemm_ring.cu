@@ -36,6 +36,7 @@ constexpr int kRows = 128, kRowBytes = 128, kTileBytes = kRows * kRowBytes;
 constexpr int kConsumers = 256, kThreads = kConsumers + 64;  // and a warp each for the weights and the activations
 constexpr int kGroupStride = kRows * 4 + 32;  // bytes of one group's scale|bias words: the next group eight banks further
 constexpr int kSumStride = kRows + 4;         // floats of one token's partial sums
+constexpr int kWeightsGaveUp = 20, kActivationsGaveUp = 21, kConsumersGaveUp = 22;  // error codes of bounded waits, none of another kernel's
 
 template <int WK, int NT>
 struct Ring {
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             if (!p.w_settled) pdl_wait();
             for (int stage = stage0, s = 0, lap = 0; stage < stage1; stage++) {
                 if (lap > 0 && !mbar_wait(empty(s), (lap - 1) & 1)) {
-                    atomicExch(err, 15);
+                    atomicExch(err, kWeightsGaveUp);
                     break;
                 }
                 mbar_expect_tx(full(s), kTileBytes + (WK ? R::KS / 64 * kRows * 4 : 0));
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         const uint16_t* xsrc = p.x + (size_t)m0 * p.ldx + q * 8;
         for (int stage = stage0, s = 0, lap = 0; stage < stage1; stage++) {
             if (lap > 0 && !__all_sync(0xffffffffu, mbar_wait(empty(s), (lap - 1) & 1))) {
-                if (lane == 0) atomicExch(err, 15);
+                if (lane == 0) atomicExch(err, kActivationsGaveUp);
                 break;
             }
             const uint16_t* src = xsrc + stage * R::KS;
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         bool alive = true;  // after a wait that ran out the sums are worthless
         for (int stage = stage0, s = 0, lap = 0, range = range0, left = range_stages; stage < stage1; stage++) {
             if (alive && !__all_sync(0xffffffffu, mbar_wait(full(s), lap & 1))) {
-                if (lane == 0) atomicExch(err, 15);
+                if (lane == 0) atomicExch(err, kConsumersGaveUp);
                 alive = false;
             }
             uint4 w[2][2];  // [half of the stage's K][row g, row g + 8]
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             // a range's sums, [token][row]: the last one over the ring, once no warp reads it any more
             uint32_t at = slots + (uint32_t)(range - range0) * R::SUMS;
             if (stage + 1 == stage1) {
-                asm volatile("bar.sync 1, %0;\n" ::"n"(kConsumers) : "memory");
+                consumers_sync();
                 at = ring;
             }
 #pragma unroll

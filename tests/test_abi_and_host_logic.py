@@ -217,3 +217,17 @@ def test_prefix_policy_restatement():
     p.store([8], 0)
     assert [e["tokens"] for e in p.entries] == [[1, 2, 3, 4, 9, 9, 9], [8]]  # [5, 6] was the least recently used
     assert p.stats == dict(lookups=4, hits=3, reused_prefix_tokens=10, computed_prefill_tokens=8)
+
+
+def test_error_codes_of_the_weight_ring_are_its_own():
+    """The code that a step reports for a wait that ran out tells the ring kernel's three roles apart, from one another and from every
+    other kernel."""
+    csrc = os.path.join(ROOT, "mlx_llm_b200", "csrc")
+    codes = {}
+    for name in sorted(os.listdir(csrc)):
+        text = open(os.path.join(csrc, name)).read()
+        constants = dict(re.findall(r"(k\w+GaveUp) = (\d+)", text))
+        for code in re.findall(r"atomicExch\([\w.]*err, (\w+)\)", text):
+            codes.setdefault(int(constants.get(code, code)), []).append(name)
+    ring = [c for c, names in codes.items() if "gemm_ring.cu" in names]
+    assert len(ring) == 3 and all(codes[c] == ["gemm_ring.cu"] for c in ring)
