@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];\n" ::"l"(&wmap) : "memory");
             if (!p.w_settled) pdl_wait();
-            for (int stage = stage0, s = 0, lap = 0; stage < stage1; stage++) {
+            int stage = stage0;
+            for (int s = 0, lap = 0; stage < stage1; stage++) {
                 if (lap > 0 && !mbar_wait(empty(s), (lap - 1) & 1)) {
                     atomicExch(err, kWeightsGaveUp);
                     break;
@@ -123,6 +124,10 @@ __global__ void __launch_bounds__(kThreads, 2)
                         bulk_load(sbring + s * R::SB_BYTES + g * kGroupStride, p.sbt + (size_t)(stage * (R::KS / 64) + g) * N + row0, kRows * 4, full(s));
                 if (++s == R::STAGES) s = 0, lap++;
             }
+            // No copy may land in shared memory that another block has by then: the consumers have waited for all of them, unless a wait
+            // of theirs ran out.
+            for (int i = max(stage0, stage - R::STAGES); i < stage; i++)
+                if (!mbar_wait(full((i - stage0) % R::STAGES), (i - stage0) / R::STAGES & 1)) break;
         }
         __syncwarp();
         pdl_wait();  // (no block may return before the kernel in front of this one has completed)
