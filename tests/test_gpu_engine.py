@@ -386,6 +386,42 @@ def test_quantize_on_load_q4_q8(env):
         H.build_engine_model(eng, ctx, H.CONFIG0, H.tiny_weights(), quant=eng.QuantSpec(64, 4))
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("matrix,silent", [("v", "o"), ("o", "v"), ("gate", "up"), ("down", "up")])
+@pytest.mark.parametrize("layer", [0, 1])
+def test_matrix_with_scales_too_large_for_a_table(env, layer, matrix, silent, bits):
+    """One weight of 2^20 gives one matrix of the model a scale that its table cannot hold.  What it is multiplied with is zero in another
+    matrix, so the logits stay ordinary numbers: those of the oracle, through the kernels for many tokens and for few."""
+    ctx, eng, orc, model, omodel = env
+    cfg = dict(H.CONFIG0, inter=640)
+    weights = H.tiny_weights(cfg, seed=5)
+    lw = weights["layers"][layer] = {k: np.array(v) for k, v in weights["layers"][layer].items()}
+    lw[matrix][(70, 9) if matrix in ("v", "gate") else (9, 70)] = 2.0 ** 20
+    group = cfg["heads"] // cfg["kv_heads"] * cfg["head_dim"]
+    if silent == "o":  # all query heads that read value row 70
+        heads = 70 // cfg["head_dim"] * group + 70 % cfg["head_dim"] + cfg["head_dim"] * np.arange(group // cfg["head_dim"])
+        lw["o"][:, heads] = 0
+    elif silent == "v":  # the value row that attention column 70 is made of
+        lw["v"][70 // group * cfg["head_dim"] + 70 % cfg["head_dim"]] = 0
+    else:
+        lw["up"][70] = 0
+    qm = H.build_engine_model(eng, ctx, cfg, weights, quant=eng.QuantSpec(64, bits))
+    om = H.build_oracle_model(orc, cfg, weights, quant_bits=bits)
+    prompts = H.config0_prompts(seed=9)[:3]
+    pool = eng.BlockPool(ctx, qm, 16, 64, 4, 16)
+    caches = [eng.PagedKvCache(pool) for _ in prompts]
+    ocs = [orc.Cache(2, block_size=16) for _ in prompts]
+    for ids in (prompts, [np.array([t], np.int32) for t in (3, 5, 7)]):
+        logits, _ = qm.step(list(zip(ids, caches)))
+        _, ref_f32 = om.forward([(p, c, c.offset()) for p, c in zip(ids, ocs)])
+        ok, err = logits_close(logits, ref_f32)
+        assert ok, f"Q{bits} logits max-abs {err}"
+    for c in caches:
+        c.free()
+    pool.free()
+    qm.free()
+
+
 def test_seeded_then_truncated_before_any_step(env):
     """A seeded cache truncated into its shared block BEFORE any forward: two block-table writes for one
     (row, index) are pending at once, and the private copy must win, or the sequence would append into a page its

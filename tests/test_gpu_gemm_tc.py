@@ -22,6 +22,16 @@ def env():
     ctx.close()
 
 
+STREAM, RING, PAIR = 1, 2, 3  # kernels that K.projection names
+
+
+def half_aligned(ctx, x):
+    """The rows of x on the device at an address that is a multiple of 8 bytes, not of 16."""
+    buf = ctx.buf(np.concatenate([np.zeros(4, np.uint16), x.ravel()]))
+    half_aligned.alive = buf  # (until the next one)
+    return buf.ptr + 8
+
+
 def quant_case(seed, n, k, bits):
     rng = np.random.default_rng(seed)
     packed = rng.integers(0, 2**32, size=(n, k * bits // 32), dtype=np.uint32)
@@ -79,15 +89,15 @@ def test_tc_matches_warp_level_kernel(env):
 
 @pytest.mark.parametrize("bits", [4, 8, 0])
 @pytest.mark.parametrize("m,n,k", [(1, 128, 256), (5, 256, 512), (8, 1024, 4096), (9, 128, 1024), (16, 384, 2048), (17, 256, 4096),
-                                   (32, 512, 1024), (3, 128, 14336)])
+                                   (32, 512, 1024), (3, 128, 14336), (2, 256, 20480)])
 def test_stream_gemm_vs_oracle(env, bits, m, n, k):
-    """Up to 32 tokens with N a multiple of 128 and K of 256 take the weight-streaming kernel: the token-tile counts
-    8, 16 and 32 wide, one and several K ranges, ragged token counts (from 33 tokens on the tcgen05 kernel takes every
-    shape its tiling fits, see test_tc_gemm_vs_oracle)."""
+    """Up to 32 tokens with N a multiple of 128 and K of 256, quantized weights without a table of scales and biases or activations
+    aligned to 8 bytes only, take the weight-streaming kernel: the token-tile counts 8, 16 and 32 wide, one and several K ranges, ragged
+    token counts (from 33 tokens on the tcgen05 kernel takes every shape its tiling fits, see test_tc_gemm_vs_oracle)."""
     ctx, K, orc, _lib = env
     rng = np.random.default_rng(7 * m + n + k)
     x = H.f32_to_bf16_np(rng.standard_normal((m, k)).astype(np.float32))
-    dx = ctx.buf(x)
+    dx = ctx.buf(x) if bits else half_aligned(ctx, x)
     yb, yf = ctx.empty((m, n), np.uint16), ctx.empty((m, n), np.float32)
     if bits:
         packed, scales, biases = quant_case(3, n, k, bits)
@@ -95,7 +105,9 @@ def test_stream_gemm_vs_oracle(env, bits, m, n, k):
         rf, _ = orc.qmm(x, packed, scales, biases, 64, bits)
     else:
         w = H.f32_to_bf16_np(rng.standard_normal((n, k)).astype(np.float32) * 0.03)
-        K.linear(ctx, dx, ctx.buf(w), m, n, k, yb, yf)
+        dw = ctx.buf(w)
+        assert K.projection(ctx, dx, dw, None, None, m, n, k, 0, y_f32=yf)[0] == STREAM
+        K.linear(ctx, dx, dw, m, n, k, yb, yf)
         rf, _ = orc.linear(x, w)
     ctx.sync()
     got = yf.download()
@@ -123,26 +135,65 @@ def test_stream_matches_tile_kernel(env):
     assert np.abs(outs[0] - outs[1]).max() <= 1e-4
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 128, 256), (8, 128, 14336), (9, 2048, 2048), (16, 384, 7936), (17, 256, 512), (31, 1024, 2048), (32, 20480, 1024), (3, 77824, 256)])
+@pytest.mark.parametrize("m,n,k", [(1, 128, 256), (8, 128, 14336), (9, 2048, 2048), (16, 384, 7936), (17, 256, 512), (31, 1024, 2048), (3, 77824, 256),
+                                   (32, 77824, 1024)])
 def test_ring_gemm_vs_oracle(env, m, n, k):
-    """Dense weights take the ring kernel up to 32 tokens: one K range and several, ranges of unequal length, blocks with several ranges,
-    clusters of every occurring size, more tiles than the machine holds at once."""
+    """Dense weights take the ring kernel up to 32 tokens: 8, 16 and 32 of them, one K range and several, more tiles than the machine
+    holds at once (clusters of every size: test_ring_gives_the_streaming_kernels_bits)."""
     ctx, K, orc, _lib = env
     rng = np.random.default_rng(m + n + k)
     x = H.f32_to_bf16_np(rng.standard_normal((m, k)).astype(np.float32))
-    w = H.f32_to_bf16_np(rng.standard_normal((n, k)).astype(np.float32) * 0.03)
+    w = H.f32_to_bf16_np(rng.standard_normal((n, k), dtype=np.float32) * np.float32(0.03))
+    dx, dw = ctx.buf(x), ctx.buf(w)
     yb, yf = ctx.empty((m, n), np.uint16), ctx.empty((m, n), np.float32)
-    K.linear(ctx, ctx.buf(x), ctx.buf(w), m, n, k, yb, yf)
+    assert K.projection(ctx, dx, dw, None, None, m, n, k, 0, y_f32=yf)[0] == RING
+    K.linear(ctx, dx, dw, m, n, k, yb, yf)
     rf, _ = orc.linear(x, w)
     ctx.sync()
     assert np.abs(yf.download() - rf).max() <= 2e-3
     assert H.close_bf16_out(yb.download(), rf)[0]
 
 
+# tokens, features, inputs, blocks per cluster, K ranges: every cluster size, one to four ranges a block, ranges of unequal length, one
+# and several rounds of blocks
+RING_PLANS = [(8, 128, 256, 1, 1), (5, 20480, 1024, 1, 2), (7, 20480, 2048, 1, 4), (2, 128, 1024, 2, 2), (16, 12288, 1536, 2, 3), (8, 128, 1536, 3, 3), (8, 6144, 3072, 3, 6),
+              (13, 128, 2048, 4, 4), (8, 5120, 4096, 4, 8), (1, 128, 2560, 5, 5), (16, 128, 5120, 5, 10), (16, 128, 3072, 6, 6), (3, 128, 6144, 6, 12),
+              (16, 128, 7168, 7, 14), (9, 128, 10240, 7, 20), (8, 128, 14336, 7, 28), (4, 128, 4096, 8, 8), (8, 128, 8192, 8, 16), (16, 128, 12288, 8, 24), (8, 128, 16384, 8, 32)]
+WIDE_RING_PLANS = [(17, 128, 256, 1, 1), (32, 77824, 1024, 1, 1), (24, 128, 1024, 2, 2), (32, 128, 1536, 3, 3), (31, 128, 2048, 4, 4), (32, 128, 2560, 5, 5),
+                   (18, 128, 3072, 6, 6), (32, 10240, 7168, 7, 7), (32, 128, 4096, 8, 8)]
+
+
+@pytest.mark.parametrize("bits,plan", [(b, p) for b in (0, 4, 8) for p in RING_PLANS] + [(b, p) for b in (0, 8) for p in WIDE_RING_PLANS])
+def test_ring_gives_the_streaming_kernels_bits(env, bits, plan):
+    """The ring kernel, dense and with a table, sums in the order of the streaming kernel, in all three epilogues."""
+    ctx, K, orc, _lib = env
+    m, n, k, cluster, ranges = plan
+    rng = np.random.default_rng(m * n + k + bits)
+    x, h = (H.f32_to_bf16_np(rng.standard_normal(s).astype(np.float32)) for s in ((m, k), (m, n)))
+    scales = biases = None
+    if bits:
+        packed, scales, biases = (ctx.buf(a) for a in quant_case(k, n, k, bits))
+    else:  # sign and mantissa at random, exponents 2^-9 to 2^-6
+        raw = rng.integers(0, 2**16, (n, k), dtype=np.uint16)
+        packed = ctx.buf((raw & 0x807f) + ((118 + (raw >> 7 & 3)) << 7).astype(np.uint16))
+    got = []
+    for dx, kernel in ((ctx.buf(x), RING), (half_aligned(ctx, x), STREAM)):
+        yb, yf, dh = ctx.empty((m, n), np.uint16), ctx.empty((m, n), np.float32), ctx.buf(h)
+        for out in (dict(y_bf16=yb), dict(y_f32=yf), dict(h=dh)):
+            route = K.projection(ctx, dx, packed, scales, biases, m, n, k, bits, **out)
+            assert route == (kernel, int(bits > 0), ranges, cluster if kernel == RING else 0)
+        ctx.sync()
+        got.append([b.download((m, n)) for b in (yb, yf, dh)])
+    assert np.isfinite(got[0][1]).all() and np.abs(got[0][1]).max() > 0.1
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("batch", [1, 8, 9, 16, 23])
 def test_ring_gemm_quantized_in_a_model(env, bits, batch):
-    """Quantized weights take the ring kernel where a model holds their table: single-token steps of a small model against the oracle."""
+    """Quantized weights take the ring kernel where a model holds their table (Q4: up to 16 tokens): single-token steps of a small model
+    against the oracle."""
     from mlx_llm_b200 import engine
     from tests.test_gpu_real_shapes import LLAMA_CUT, run_schedule
 
@@ -163,7 +214,7 @@ def double_rounded(codes, scales, biases):
     return twice, H.f32_to_bf16_np(sticky.view(np.float32))
 
 
-@pytest.mark.parametrize("m,kernel", [(8, 2), (16, 2), (32, 2), (512, 3)])
+@pytest.mark.parametrize("m,kernel", [(8, RING), (16, RING), (32, RING), (512, PAIR)])
 def test_q8_weights_are_rounded_as_dequantize_does(env, m, kernel):
     """Both kernels that read the table of scales and biases make the weights of b2_dequantize bit for bit, also where a bias far below
     its scale decides a tie: an identity matrix as activations reads the weights out."""
@@ -213,7 +264,7 @@ def test_weights_that_the_call_before_wrote(env, rows):
     for turn in range(12):
         for at, source in enumerate(sources[turn & 1]):
             K.linear(ctx, source, a, rows, k, inner, y_bf16=w.ptr + at * rows * k * 2)
-        x_at = x.ptr + (8 if turn & 2 else 0)
+        x_at = x.ptr + (8 if turn & 2 else 0)  # (the streaming kernel, the ring kernel)
         K.linear(ctx, x_at, w, 8, n, k, y_f32=outs[0])
         ctx.sync()
         K.linear(ctx, x_at, w, 8, n, k, y_f32=outs[1])  # (nothing in flight any more)
@@ -253,7 +304,7 @@ def test_table_of_any_size_of_scales(env, name, m, bits):
     dx, dp, ds, db = ctx.buf(x), ctx.buf(packed), ctx.buf(scales), ctx.buf(biases)
     with_table, without = ctx.empty((m, n), np.float32), ctx.empty((m, n), np.float32)
     route = K.projection(ctx, dx, dp, ds, db, m, n, k, bits, y_f32=with_table)
-    assert route[:2] == (3 if m > 32 else 2 if possible else 1, int(possible))
+    assert route[:2] == (PAIR if m > 32 else RING if possible else STREAM, int(possible))
     K.qmm(ctx, dx, dp, ds, db, m, n, k, bits, None, without)
     ctx.sync()
     want = without.download()
