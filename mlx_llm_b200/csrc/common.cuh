@@ -29,6 +29,14 @@ int32_t b2_fail(int32_t code, const std::string& msg);
         if (!(cond)) return b2_fail((code), (msg)); \
     } while (0)
 
+// Function of the CUDA driver, null where it has none of that name (the library links the runtime alone).
+template <typename Fn>
+inline Fn b2_driver_fn(const char* name) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Fn>(fn) : nullptr;
+}
+
 // ---- context --------------------------------------------------------------------------------
 struct b2_ctx {
     int device = 0;

@@ -93,17 +93,11 @@ int32_t ensure_workspace(b2_model* m, int T, int B, int W, int P, size_t stage_i
     return B2_OK;
 }
 
-template <typename Fn>
-Fn driver_fn(const char* name) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    return cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Fn>(fn) : nullptr;
-}
 // True when [p, p + bytes) lies in one allocation of page-locked host memory: the copy engine can then write a result there
 // itself.  Memory that was only registered does not count (it may be registered for reading alone).
 bool pinned_range(void* p, size_t bytes) {
-    static const auto attribute = driver_fn<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>("cuPointerGetAttribute");
-    static const auto host_flags = driver_fn<CUresult (*)(unsigned*, void*)>("cuMemHostGetFlags");
+    static const auto attribute = b2_driver_fn<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>("cuPointerGetAttribute");
+    static const auto host_flags = b2_driver_fn<CUresult (*)(unsigned*, void*)>("cuMemHostGetFlags");
     unsigned type = 0, flags = 0;
     CUdeviceptr start = 0;
     size_t size = 0;
