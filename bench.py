@@ -104,7 +104,7 @@ NCU_TRAFFIC = {
     "gemm_gate_up": dict(kernel="gemm_tc_pair_kernel<4,0>", bytes_per_launch=94.1e6, summary="gemm_tc_pair_kernel_q4_2layer_step.md",
                          note="gate+up projection launch (N 28672, K 4096) at ~570 tokens in the 2-layer capture; algorithmic 66.1 MB of packed "
                               "weights + activations/outputs that mostly stay in L2"),
-    "paged_attn_decode_config1": dict(kernel="paged_attn_decode_kernel<128>", bytes_per_launch=572.7e6, summary="paged_attn_decode_kernel_config1.md",
+    "paged_attn_decode_config1": dict(kernel="paged_attn_decode_kernel<128, 2>", bytes_per_launch=572.7e6, summary="paged_attn_decode_kernel_config1.md",
                                       note="the configuration-1 batch (algorithmic 565.0 MB)"),
     "gemm_stream_gate_up": dict(kernel="gemm_stream_kernel<4,1,0>", bytes_per_launch=66.2e6, summary="gemm_stream_kernel_decode_only_step.md",
                                 note="gate+up projection (28672 x 4096, Q4) at 8 tokens in a decode-only iteration; algorithmic 66.1 MB"),
@@ -400,7 +400,7 @@ def run_paged_attn(args, rank, world, local_rank, barrier, reduce_max, reduce_su
                     l2="flushed between timed iterations", parallelism=f"replica x{world}", chunk_tokens=args.chunk_tokens or 512),
         roofline=dict(bound="hbm", achieved=gbs, peak=peaks["hbm_gbs"], unit="GB/s", frac=gbs / peaks["hbm_gbs"],
                       traffic=ncu_traffic("paged_attn_decode_config1")[0], traffic_note=ncu_traffic("paged_attn_decode_config1")[1],
-                      peak_source=peaks["source"], algorithmic_bytes=alg, kernel="paged_attn_decode_kernel<128> (work list and merge inside: one launch)",
+                      peak_source=peaks["source"], algorithmic_bytes=alg, kernel="paged_attn_decode_kernel<128, 2> (work list and merge inside: one launch)",
                       unflushed=dict(ms_per_step=t_unflushed / args.steps, achieved=alg / (t_unflushed / args.steps * 1e-3) / 1e9,
                                      frac=alg / (t_unflushed / args.steps * 1e-3) / 1e9 / peaks["hbm_gbs"],
                                      note="the same iterations back to back, no flush: the inputs (565 MB of a 1.1 GB pool per iteration) exceed L2")),
@@ -617,7 +617,7 @@ def run_decode_only(args, rank, world, local_rank, barrier, reduce_max, reduce_s
                     parallelism=f"replica x{world}", l2="every iteration streams 5 GB of weights, far beyond L2",
                     generated_tokens_per_step=gen / max(steps, 1)),
         roofline=dict(bound="hbm", achieved=gbs, peak=peaks["hbm_gbs"], unit="GB/s", frac=gbs / peaks["hbm_gbs"], traffic=None,
-                      peak_source=peaks["source"], kernel="gemm_stream_kernel (projection weights once per iteration) + bf16 lm_head",
+                      peak_source=peaks["source"], kernel="gemm_ring_kernel up to 16 sequences, gemm_tc_pair_kernel from 33 (projection weights once per iteration) + bf16 lm_head",
                       algorithmic_bytes_per_step=weight_bytes, ms_per_step=gemm_ms, launches_per_step=prof["launches"]["gemm"] / prof_steps),
         class_ms_per_step={k: v / prof_steps for k, v in prof["ms"].items()},
         e2e=dict(value=all_gen / (all_wall * 1e-3), unit="tok/s", h2d_bytes_per_step=int((s1["h2d_bytes"] - st["h2d_bytes"]) / max(steps, 1)),

@@ -4,7 +4,7 @@
 //
 // Same contract as the register-streaming kernel in gemm_stream.cu (primitives::nn::linear, src/primitives/nn.rs:26-33;
 // QuantizedLinear::forward, src/primitives/quant.rs:56-70): the weights are the A operand of mma.sync m16n8k16, dequantised in
-// registers with one rounding, the tokens its 8-wide N side.  HBM bounds these calls, and behind it the instructions that a weight
+// registers to that kernel's weights, the tokens its 8-wide N side.  HBM bounds these calls, and behind it the instructions that a weight
 // costs and the fixed time of a launch.
 //   * A stage, 128 feature rows x 128 bytes, comes in by one TMA copy, with its scales and biases (from the transposed table) as bulk
 //     copies on the same barrier: no address arithmetic, no load per row, 130 KB in flight on an SM without a register.
@@ -17,10 +17,10 @@
 //     that kernel writes partial sums to global memory and lets the block that counts in last read them back.
 // The weights of a model do not depend on the kernel before this one: the ring is filled with them before the wait for that kernel.
 // One token, us a call among others of its kind, register-streaming kernel -> this one (bytes at the copy rate): 28672 x 4096 Q4
-// 28.8 -> 22.7 (10.2), 4096 x 14336 Q4 17.6 -> 14.7 (5.1), 51200 x 5120 Q8 100 -> 50.4 (43.1), 5120 x 25600 Q8 55.1 -> 28.2 (21.6),
-// 2048 x 2048 bf16 7.2 -> 5.0 (1.3), 128256 x 4096 bf16 173 -> 160 (163); 16 tokens: 39.9 -> 33.1, 25.8 -> 19.8, 112 -> 58.5,
-// 67.1 -> 35.7, 9.2 -> 6.0, 185 -> 170.  With 17 to 32 tokens on Q4 the activations leave the ring too few stages, and the other
-// kernel is faster; on Q8 and bf16 it is not (32 tokens: 51200 x 5120 Q8 128 -> 79, 28672 x 4096 bf16 62 -> 55).
+// 29.1 -> 22.3 (10.2), 4096 x 14336 Q4 17.4 -> 14.4 (5.1), 51200 x 5120 Q8 100 -> 52.1 (43.1), 5120 x 25600 Q8 55.2 -> 29.3 (21.6),
+// 2048 x 2048 bf16 7.1 -> 5.1 (1.3), 128256 x 4096 bf16 172 -> 159 (163); 16 tokens: 39.6 -> 32.8, 25.5 -> 19.9, 112 -> 63.4,
+// 67.1 -> 36.6, 9.2 -> 6.1, 185 -> 170.  With 17 to 32 tokens on Q4 the activations leave the ring too few stages, and the other
+// kernel is faster; on Q8 and bf16 it is not (32 tokens: 51200 x 5120 Q8 127 -> 80, 28672 x 4096 bf16 62 -> 55).
 #include <atomic>
 #include <type_traits>
 
@@ -310,7 +310,7 @@ int max_clusters(b2_ctx* ctx, int splits) {
 
 // Blocks of a cluster that share a row tile's K: 0 where a block would have more ranges than it has room for.  The cost is in stages
 // of an SM's time: two blocks there share it, one alone takes 3/4 as long as the two; a round of blocks costs some 14 more.  One token,
-// us with clusters of 1 .. 8 (- : too many ranges a block):
+// us with clusters of 1 .. 8 (- : too many ranges a block; Q8 with weights rounded once throughout, 4 % below now):
 //   4096 x 14336 Q4   - - - - 17.1 16.3 14.7 14.8      5120 x 25600 Q8  - - - 34.6 28.2 29.5 40.1 38.3      6144 x 4096 Q4  - 9.0 9.8 8.4 8.5 12.8 13.2 11.3
 //   28672 x 4096 Q4   22.7 29.3 26.5                   51200 x 5120 Q8  57.0 50.4                           10240 x 5120 Q8  - 16.0 13.4 20.1 19.7 19.3 22.5
 //   17792 x 2048 bf16 14.9 14.0 19.2 16.3              28672 x 4096 bf16  39.4 44.1 44.2                    2048 x 2048 bf16  10.4 6.8 6.8 5.0
