@@ -93,17 +93,20 @@ int32_t ensure_workspace(b2_model* m, int T, int B, int W, int P, size_t stage_i
     return B2_OK;
 }
 
-// True when [p, p + bytes) lies in one allocation of page-locked host memory: the copy engine can then write a result there
-// itself.  Memory that was only registered does not count (it may be registered for reading alone).
+// True when [p, p + bytes) lies in one allocation of page-locked host memory that kernels reach at the same address: a kernel can then
+// write a result there itself.  Memory that was only registered does not count (it may be registered for reading alone), nor does
+// write-combined memory.
 bool pinned_range(void* p, size_t bytes) {
     static const auto attribute = b2_driver_fn<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>("cuPointerGetAttribute");
     static const auto host_flags = b2_driver_fn<CUresult (*)(unsigned*, void*)>("cuMemHostGetFlags");
     unsigned type = 0, flags = 0;
-    CUdeviceptr start = 0;
+    CUdeviceptr start = 0, seen = 0;
     size_t size = 0;
     const CUdeviceptr at = (CUdeviceptr)(uintptr_t)p;
     return attribute && host_flags && attribute(&type, CU_POINTER_ATTRIBUTE_MEMORY_TYPE, at) == CUDA_SUCCESS && type == CU_MEMORYTYPE_HOST &&
-           host_flags(&flags, p) == CUDA_SUCCESS && attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) == CUDA_SUCCESS &&
+           host_flags(&flags, p) == CUDA_SUCCESS && (flags & CU_MEMHOSTALLOC_WRITECOMBINED) == 0 &&
+           attribute(&seen, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, at) == CUDA_SUCCESS && seen == at &&
+           attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) == CUDA_SUCCESS &&
            attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) == CUDA_SUCCESS && at >= start && at - start <= size && bytes <= size - (at - start);
 }
 
@@ -484,16 +487,13 @@ int32_t b2_engine_forward(b2_model* m, std::vector<SeqStep>& seqs, void* logits_
         B2_CHECK(forward_bf16_layers(m, pool, mo, in, ids_dev, T, n_dec, dec_ctx_sum, W, P, pf_flops, pf_max_ctx, chunk_tiles, q_tile, n_logits, logit_rows));
     }
     const int lsz = m->logits_f32() ? 4 : 2;
-    // Logits go straight into a page-locked buffer of the caller, once the step is known to be whole; a pageable one gets them through a
+    // Logits go straight into a page-locked buffer of the caller, unless the step is abandoned; a pageable one gets them through a
     // page-locked buffer of the model.  The host's copy between the two was 0.6 ms of a 64-sequence step (128256 bf16 logits each),
     // 0.9 ms of a 97-sequence one.
     const size_t logits_bytes = (size_t)n_logits * c.vocab_size * lsz;
     const bool direct = logits_out && logits_bytes && pinned_range(logits_out, logits_bytes);
-    auto copy_logits = [&](void* to) {
-        m->d2h_bytes += (int64_t)logits_bytes;
-        return cudaMemcpy2DAsync(to, (size_t)c.vocab_size * lsz, m->logits_f32() ? (const void*)logits_f32_dev : (const void*)w.logits,
-                                 (size_t)logits_ld * lsz, (size_t)c.vocab_size * lsz, (size_t)n_logits, cudaMemcpyDeviceToHost, st);
-    };
+    const void* logits_dev = m->logits_f32() ? (const void*)logits_f32_dev : (const void*)w.logits;
+    const size_t logits_pitch = (size_t)logits_ld * lsz, logits_width = (size_t)c.vocab_size * lsz;
     if (n_logits > 0) {
         b2_prof_mark(ctx, B2_CLS_META);
         B2_CUDA(cudaMemcpyAsync(w.argmax_host, w.argmax, (size_t)n_logits * 4, cudaMemcpyDeviceToHost, st));
@@ -505,24 +505,23 @@ int32_t b2_engine_forward(b2_model* m, std::vector<SeqStep>& seqs, void* logits_
                 B2_CUDA(cudaHostAlloc((void**)&w.logits_host, logits_bytes, cudaHostAllocDefault));
                 w.logits_host_cap = logits_bytes;
             }
-            B2_CUDA(copy_logits(w.logits_host));
+            B2_CUDA(cudaMemcpy2DAsync(w.logits_host, logits_width, logits_dev, logits_pitch, logits_width, (size_t)n_logits, cudaMemcpyDeviceToHost, st));
+            m->d2h_bytes += (int64_t)logits_bytes;
         }
     }
     // the error word a bounded device-side wait raises travels back with the sampled ids
     B2_CUDA(cudaMemcpyAsync(ctx->err_host, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     m->d2h_bytes += (int64_t)sizeof(int);
-    b2_prof_mark(ctx, -1);
-    B2_CUDA(cudaEventRecord(m->ev1, st));
-    B2_CUDA(cudaStreamSynchronize(st));
-    if (direct && ctx->err_host[0] == 0) {
-        b2_prof_mark(ctx, B2_CLS_META);
-        const cudaError_t copied = copy_logits(logits_out);
-        b2_prof_mark(ctx, -1);
-        const cudaError_t marked = cudaEventRecord(m->ev1, st);
-        B2_CUDA(cudaStreamSynchronize(st));  // (before anything may return: the buffer is the caller's)
-        B2_CUDA(copied);
-        B2_CUDA(marked);
+    int32_t copied = B2_OK;
+    if (direct) {
+        copied = b2_rows_to_host_launch(ctx, logits_dev, logits_pitch, logits_out, logits_width, n_logits);
+        m->d2h_bytes += (int64_t)logits_bytes;
     }
+    b2_prof_mark(ctx, -1);
+    const cudaError_t marked = cudaEventRecord(m->ev1, st);
+    B2_CUDA(cudaStreamSynchronize(st));  // (before anything else returns: the buffer is the caller's)
+    B2_CHECK(copied);
+    B2_CUDA(marked);
     B2_CUDA(cudaGetLastError());
     b2_prof_collect(ctx);
     float ms = 0.f;

@@ -4,6 +4,7 @@
 // Rounding points follow the reference, where every MLX op materialises a bf16 tensor
 // (src/models/llama.rs:718-735, :1040-1045): reductions run in f32, each op's result is rounded to
 // bf16 once.
+#include <algorithm>
 #include <cfloat>
 
 #include "common.cuh"
@@ -220,6 +221,16 @@ int32_t launch_argmax(b2_ctx* ctx, const T* logits, int64_t ld, int rows, int vo
     return B2_OK;
 }
 
+// Rows into page-locked host memory, unless a bounded wait of the step has run out: what the caller's buffer holds then stays, and the
+// host need not wait for the error word before it asks for the copy (15 us a step).  Bound by PCIe.
+template <typename U>
+__global__ void __launch_bounds__(512) rows_to_host_kernel(const U* __restrict__ src, size_t ld, U* __restrict__ dst, size_t width, const int* __restrict__ err) {
+    if (*err != 0) return;
+    const U* s = src + blockIdx.y * ld;
+    U* d = dst + blockIdx.y * width;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < width; i += (size_t)gridDim.x * blockDim.x) d[i] = s[i];
+}
+
 // Standalone dequantize / unpack of the MLX affine format (src/primitives/quant.rs:73-82).
 __global__ void dequantize_kernel(const uint32_t* __restrict__ packed, const uint16_t* __restrict__ scales,
                                   const uint16_t* __restrict__ biases, int64_t total_words, int64_t words_per_row, int64_t groups,
@@ -334,6 +345,30 @@ int32_t b2_residual_add_f32_launch(b2_ctx* ctx, const float* y, int64_t n, uint1
     const int64_t quads = (n + 3) / 4;
     residual_add_f32_kernel<<<(unsigned)((quads + 255) / 256), 256, 0, ctx->stream>>>(y, n, x);
     B2_LAUNCHED(ctx);
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
+template <typename U>
+static void launch_rows_to_host(b2_ctx* ctx, const void* src, size_t ld, void* dst, size_t width, int rows) {
+    const dim3 grid((unsigned)std::min<size_t>((width / sizeof(U) + 511) / 512, 64), (unsigned)rows);
+    rows_to_host_kernel<U><<<grid, 512, 0, ctx->stream>>>((const U*)src, ld / sizeof(U), (U*)dst, width / sizeof(U), ctx->dev_err);
+}
+int32_t b2_rows_to_host_launch(b2_ctx* ctx, const void* src, size_t ld, void* dst, size_t width, int rows) {
+    const size_t all = (size_t)(uintptr_t)src | ld | (size_t)(uintptr_t)dst | width;
+    for (int row = 0; row < rows; row += 65535) {  // (grid.y)
+        const void* s = (const uint8_t*)src + row * ld;
+        void* d = (uint8_t*)dst + row * width;
+        const int n = std::min(rows - row, 65535);
+        if (all % 16 == 0)
+            launch_rows_to_host<uint4>(ctx, s, ld, d, width, n);
+        else if (all % 4 == 0)
+            launch_rows_to_host<uint32_t>(ctx, s, ld, d, width, n);
+        else if (all % 2 == 0)
+            launch_rows_to_host<uint16_t>(ctx, s, ld, d, width, n);
+        else
+            launch_rows_to_host<uint8_t>(ctx, s, ld, d, width, n);
+        B2_LAUNCHED(ctx);
+    }
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }

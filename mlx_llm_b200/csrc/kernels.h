@@ -115,6 +115,8 @@ int32_t b2_add_launch(b2_ctx* ctx, const uint16_t* a, const uint16_t* b, int64_t
 // x = bf16(x + bf16(y)), y f32 (n a multiple of 4 for the vector path; any n works)
 int32_t b2_residual_add_f32_launch(b2_ctx* ctx, const float* y, int64_t n, uint16_t* x);
 // Greedy argmax per row over bf16 logits, ties -> lowest index.
+// `rows` rows of `width` bytes, `ld` bytes apart, into page-locked host memory one after the other; nothing where the context's error word is set.
+int32_t b2_rows_to_host_launch(b2_ctx* ctx, const void* src, size_t ld, void* dst, size_t width, int rows);
 int32_t b2_argmax_launch(b2_ctx* ctx, const uint16_t* logits, int rows, int vocab, int32_t* out);
 int32_t b2_dequantize_launch(b2_ctx* ctx, const uint32_t* packed, const uint16_t* scales, const uint16_t* biases, int64_t rows,
                              int64_t in_dim, int bits, uint16_t* out);
